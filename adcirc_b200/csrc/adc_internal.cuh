@@ -200,17 +200,25 @@ struct adc_ctx {
   adc::Bar *bar;
   void *jlines;          // JCG barrier lines: 2 x 128 B per row block
   int jcg_grid, jcg_rows_blocks;
-  // JCG resident variant (block-local indices, halo lists, export flags)
-  int jcg_res, jcg_rows_max, jcg_halo_max, jcg_stage_bytes, jcg_stage_wcap;
+  // JCG resident kernel (block-local columns, halo lists, row lengths)
+  int jcg_res;                 // 0: jcg_kernel, 1: resident on the grid, 2: in one cluster,
+                               // 3: jcg_ordered_kernel
+  int jcg_res_k, jcg_rows_max, jcg_halo_max, jcg_stage_bytes;
+  int jr_o[9];                 // its shared-memory offsets
   size_t jcg_smem;
+  int jcg_stage_wcap;
+  unsigned char *jtab;         // one allocation behind the tables below
   unsigned short *jlcol;
+  uint4 *jrcol;
+  int4 *jmeta;
+  unsigned char *jrle;
   float *soff32;               // FP32 scaled matrix (mixed mode, resident variant)
   double *etas_prev;           // last step's reference guess (ADC_WARM_START)
   WarmState *warm;
   adc::Mpnn *mp;               // learned initial guess (mpnn.cu), built on first use
   int *h_neitab, *h_nneigh;    // host copies of NeiTab/NNeigh (the predictor's 1-ring)
-  int *jhalo_ptr, *jhalo_ids;
-  unsigned char *jexp;
+  int *jhalo_ptr, *jhalo_ids, *jpush_ptr;
+  int2 *jpush;
   // flags / steps
   adc::Flags *flags;
   adc_step_t *steps;     // device step table
@@ -261,6 +269,7 @@ int launch_shift_friction(adc_ctx *c);
 int launch_gwce_lhs(adc_ctx *c);
 int launch_gwce_rhs(adc_ctx *c);
 int launch_jcg(adc_ctx *c, int eta_update);
+void jcg_clear_barrier(adc_ctx *c);
 int launch_wetdry(adc_ctx *c);
 int launch_momentum(adc_ctx *c);
 

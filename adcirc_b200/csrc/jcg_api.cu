@@ -30,9 +30,8 @@ struct Stage {
   adc_ctx c;
   Stage() { memset((void *)&c, 0, sizeof(c)); }
   ~Stage() {
-    void *ptrs[] = {c.sl_ptr, c.sl_w, c.col, c.rlen, c.offd, c.soff, c.diag, c.gwce_lv,
-                    c.etas, c.ju1, c.jp[0], c.jp[1], c.jw, c.jexp, c.jlcol, c.jhalo_ptr, c.jhalo_ids,
-                    c.jpart, c.jtri, c.itp, c.bar, c.flags, c.jlines};
+    void *ptrs[] = {c.sl_ptr, c.sl_w, c.col, c.rlen, c.offd, c.soff, c.diag, c.gwce_lv, c.etas, c.ju1,
+                    c.jp[0], c.jp[1], c.jw, c.jtab, c.itp, c.bar, c.flags, c.jlines};
     for (void *p : ptrs)
       if (p) cudaFree(p);
     if (c.stream) cudaStreamDestroy(c.stream);
@@ -114,9 +113,8 @@ static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, doubl
   const JcgHostSell hs{sl_ptr.data(), sl_w.data(), col.data(), rlen.data()};
   int rc = jcg_setup_grid(&c, &hs);
   if (rc) return rc;
-  ADC_CUDA(alloc_up<double>(&c.jpart, nullptr, 4 * (size_t)c.jcg_grid));
-  ADC_CUDA(alloc_up<double>(&c.jtri, nullptr, 4 * (size_t)std::max(itmax, 2)));
   ADC_CUDA(alloc_up<char>((char **)&c.jlines, nullptr, 2 * 128 * (size_t)c.jcg_rows_blocks));
+  jcg_clear_barrier(&c);
   Itp it;
   memset(&it, 0, sizeof(it));
   it.zeta = rparm[0];

@@ -476,8 +476,8 @@ static void free_ctx(adc_ctx *c) {
       (void **)&c->bc_row, (void **)&c->ebuf,
       (void **)&c->ebuf2, (void **)&c->red, (void **)&c->ev_cnt, (void **)&c->ev_a,
       (void **)&c->ev_b, (void **)&c->ev_c, (void **)&c->evu_i, (void **)&c->evu_c, (void **)&c->ju1, (void **)&c->jp[0],
-      (void **)&c->jp[1], (void **)&c->jw, (void **)&c->jexp, (void **)&c->jlcol,
-      (void **)&c->jhalo_ptr, (void **)&c->jhalo_ids, (void **)&c->soff32, (void **)&c->etas_prev, (void **)&c->warm, (void **)&c->soff, (void **)&c->jpart, (void **)&c->jtri,
+      (void **)&c->jp[1], (void **)&c->jw, (void **)&c->jtab,
+      (void **)&c->soff32, (void **)&c->etas_prev, (void **)&c->warm, (void **)&c->soff,
       (void **)&c->itp, (void **)&c->bar, (void **)&c->jlines, (void **)&c->flags, (void **)&c->steps,
       (void **)&c->numitr_log, (void **)&c->met_wsx, (void **)&c->met_wsy,
       (void **)&c->met_pr, (void **)&c->vfix, (void **)&c->vstate, (void **)&c->eser,
@@ -651,10 +651,9 @@ static int bind_impl(const adc_params_t *p, const adc_arrays_t *a, int prec, adc
     const JcgHostSell hs{T.sl_ptr.data(), T.sl_w.data(), T.col.data(), T.rlen.data()};
     B(jcg_setup_grid(c, &hs));
   }
-  B(dalloc(&c->jpart, 4 * (size_t)c->jcg_grid));
-  B(dalloc(&c->jtri, 4 * (size_t)std::max(c->itmax, 2)));
   B(dalloc(&c->itp, 1)); B(dalloc(&c->bar, 1));
   B(dalloc((char **)&c->jlines, 2 * 128 * (size_t)c->jcg_rows_blocks));
+  jcg_clear_barrier(c);
   {
     // Flags followed by the rebuild word.
     char *f = nullptr;
@@ -969,8 +968,7 @@ int adc_set_jcg_blocks(adc_ctx *c, int nrb) {
   if (!c || nrb < 0) return ADC_ERR_ARG;
   ADC_CUDA(cudaStreamSynchronize(c->stream));
   drop_graphs(c);
-  void **old[] = {(void **)&c->jlcol, (void **)&c->jhalo_ptr, (void **)&c->jhalo_ids,
-                  (void **)&c->jexp, (void **)&c->jpart, (void **)&c->jlines};
+  void **old[] = {(void **)&c->jtab, (void **)&c->jlines};
   for (void **q : old)
     if (*q) { cudaFree(*q); *q = nullptr; }
   const size_t nsl = c->nslices, nnz = c->nnz_pad;
@@ -982,15 +980,19 @@ int adc_set_jcg_blocks(adc_ctx *c, int nrb) {
   c->jcg_nrb_req = nrb;
   const JcgHostSell hs{sl_ptr.data(), sl_w.data(), col.data(), rlen.data()};
   TRY(jcg_setup_grid(c, &hs));
-  TRY(dalloc(&c->jpart, 4 * (size_t)c->jcg_grid));
   TRY(dalloc((char **)&c->jlines, 2 * 128 * (size_t)c->jcg_rows_blocks));
+  jcg_clear_barrier(c);
+  // no exchange word of the old layout may pass for one of the new
+  ADC_CUDA(cudaMemsetAsync(c->jp[0], 0, nsl * kSlice * sizeof(double4), c->stream));
+  ADC_CUDA(cudaMemsetAsync(c->jp[1], 0, nsl * kSlice * sizeof(double4), c->stream));
+  ADC_CUDA(cudaStreamSynchronize(c->stream));
   return ADC_OK;
 }
 
 int adc_jcg_layout(adc_ctx *c, int *row_blocks, int *resident) {
   if (!c) return ADC_ERR_ARG;
   if (row_blocks) *row_blocks = c->jcg_rows_blocks;
-  if (resident) *resident = c->jcg_res;
+  if (resident) *resident = c->jcg_res != 0;
   return ADC_OK;
 }
 
