@@ -221,6 +221,7 @@ struct adc_ctx {
   int2 *jpush;
   // flags / steps
   adc::Flags *flags;
+  int *tickets;          // blocks done, of the kernels whose last block ends a pass
   adc_step_t *steps;     // device step table
   int steps_cap;
   int *numitr_log;
@@ -265,13 +266,23 @@ int cuda_fail(cudaError_t e, const char *what);
 inline int nblk(long long n, int t = kThreads) { return (int)((n + t - 1) / t); }
 
 // Phase launchers (each returns ADC_OK or an error, records launches).
-int launch_shift_friction(adc_ctx *c);
-int launch_gwce_lhs(adc_ctx *c);
-int launch_gwce_rhs(adc_ctx *c);
-int launch_jcg(adc_ctx *c, int eta_update);
+int launch_shift_friction(adc_ctx *c, bool whole);
+int launch_gwce(adc_ctx *c);
+int launch_jcg(adc_ctx *c, int eta_update, bool d1);
 void jcg_clear_barrier(adc_ctx *c);
-int launch_wetdry(adc_ctx *c);
-int launch_momentum(adc_ctx *c);
+int launch_wetdry(adc_ctx *c, bool whole, bool d1_done);
+int launch_momentum(adc_ctx *c, bool whole, int *log);
+
+// D1 of the wet/dry pass for one node (wetdry.F:234-285): whether a wet node
+// dries; ETA2 is raised to leave at least 0.8 H0 of water.
+__device__ __forceinline__ bool d1_dries(int nodecode, double dp, double h0, double &eta2) {
+  if (nodecode != 1) return false;
+  const double htot = dp + eta2;
+  if (!(htot <= h0)) return false;
+  const double habsmin = 0.8 * h0;
+  if (htot < habsmin) eta2 = habsmin - dp;
+  return true;
+}
 
 // Drops the captured step graphs (after a change they would not see).
 inline void drop_graphs(adc_ctx *c) {

@@ -23,7 +23,7 @@
 //    here one thread per boundary node adds its contributions in that same
 //    order (a table built at bind lists them), so GWCE_LV gets the same bits;
 //  * the specified normal velocity -QN2/H2 of the momentum boundary
-//    conditions (momentum.F:815-856), read in k_mom_node; radiation nodes
+//    conditions (momentum.F:815-856), read in node_mom; radiation nodes
 //    take no momentum boundary condition.
 // External barriers (IBTYPE 3/13/23) take as QN2 the free-surface
 // supercritical outflow over the crest once the water stands BARMIN above it
@@ -42,10 +42,10 @@
 // 2469-2579, timestep.F:1034-1044).
 // It also holds the non-periodic boundary series: fort.20 fluxes in place of
 // the periodic constituents (NFFR <= 0, timestep.F:882-903) and fort.19
-// elevations added to the periodic boundary elevation in k_eta_bc
-// (gwce.F:1659-1674).  Both files sit whole in HBM; k_series_state moves
+// elevations added to the periodic boundary elevation in bnd_eta
+// (gwce.F:1659-1674).  Both files sit whole in HBM; one_series moves
 // the pair of record times as the reference's reads do.
-#include "adc_internal.cuh"
+#include "step_bodies.cuh"
 
 #include <cmath>
 #include <cstring>
@@ -53,233 +53,51 @@
 
 namespace adc {
 
-// One thread: per active series, the record pair and ratio of this step.
-// The reference reads the next record when TimeLoc passes the later record
-// time, at most once per step (gwce.F:1660-1668, timestep.F:882-900).
-__global__ void k_series_state(adc_ctx c, const adc_step_t *steps, Flags *flags) {
+__global__ void k_series_state(adc_ctx c, const adc_step_t *steps) {
   griddep_wait();
-  const double timeloc = steps[flags->cursor].timeloc;
-  for (int s = 0; s < 2; ++s) {
-    if (!(s == 0 ? c.eser_on : c.fser_on)) continue;
-    SeriesState &st = c.sstate[s];
-    const int nrec = s == 0 ? c.eser_nrec : c.fser_nrec;
-    const double inc = s == 0 ? c.eser_interval : c.fser_interval;
-    if (timeloc > st.t2) {
-      st.t1 = st.t2;
-      st.t2 = st.t1 + inc;
-      st.k = st.k + 1;
-      if (st.k + 1 >= nrec) {   // the file has no further record
-        st.err = 1;
-        flags->status = ADC_ERR_ARG;
-        st.k = nrec - 2;
-      }
-    }
-    st.ratio = (timeloc - st.t1) / inc;
-  }
+  one_series(c, steps[c.flags->cursor].timeloc);
 }
 
-// COMPUTE_INTERNAL_BOUNDARY_FLUX (weir_boundary.F90:1775-1942, the default
-// wet-edge formulation without averaging); the square roots stand for the
-// reference's **0.5.
-__device__ double internal_barrier_flux(const adc_ctx &c, int I, double ramp) {
-  const int n1 = c.bnv[I], n2 = c.ibconn[I], kind = c.ibkind[I];
-  const int *nc = c.nodecode;
-  int wn1 = 0, wn2 = 0;   // wet neighbours along the barrier on each side
-  if (kind == 0) {
-    wn1 = wn1 + nc[c.bnv[I + 1]];
-    wn2 = wn2 + nc[c.ibconn[I + 1]];
-  } else if (kind == 1) {
-    wn1 = wn1 + nc[c.bnv[I - 1]];
-    wn2 = wn2 + nc[c.ibconn[I - 1]];
-  } else {
-    wn1 = wn1 + nc[c.bnv[I - 1]];
-    wn1 = wn1 + nc[c.bnv[I + 1]];
-    wn2 = wn2 + nc[c.ibconn[I + 1]];
-    wn2 = wn2 + nc[c.ibconn[I - 1]];
-  }
-  const double R1 = c.eta2[n1] - c.binht[I], R2 = c.eta2[n2] - c.binht[I];
-  const double R1F = 2.0 * R1 / 3.0, R2F = 2.0 * R2 / 3.0;
-  const double G = c.p.g, BARMIN = 0.04;
-  double flux = 0.0;
-  if ((R1 < 0.0) && (R2 < 0.0)) {
-    flux = 0.0;
-  } else if (fabs(R1 - R2) < 0.01) {
-    flux = 0.0;
-  } else if ((R1 > R2) && (R1 > BARMIN)) {   // this side is the source
-    if (nc[n1] == 0 || wn1 == 0) flux = 0.0;
-    else if (R2 > R1F) flux = -ramp * R2 * c.bincfsb[I] * sqrt(2.0 * G * (R1 - R2));
-    else flux = -ramp * c.bincfsp[I] * R1F * sqrt(R1F * G);
-  } else if ((R2 > R1) && (R2 > BARMIN)) {   // this side receives
-    if (nc[n2] == 0 || wn2 == 0) {
-      flux = 0.0;
-    } else {
-      if (R1 > R2F) flux = ramp * R1 * c.bincfsb[I] * sqrt(2.0 * G * (R2 - R1));
-      else flux = ramp * c.bincfsp[I] * R2F * sqrt(R2F * G);
-      c.nib[n1] = 1;
-    }
-  }
-  return flux;
-}
-
-// COMPUTE_CROSS_BARRIER_PIPE_FLUX (weir_boundary.F90:2469-2579); the
-// reference's **0.5 as square roots and PIPEDIAM**2 as a product.
-__device__ double pipe_flux(const adc_ctx &c, int I, double ramp) {
-  const int n1 = c.bnv[I], n2 = c.ibconn[I];
-  const double *pp = c.pipe;
-  const double ht = pp[I], coef = pp[c.nvel + I], diam = pp[2 * c.nvel + I];
-  const double G = c.p.g, BARMIN = 0.04, PI = 3.141592653589793;
-  const double R1 = c.eta2[n1] - ht, R2 = c.eta2[n2] - ht;
-  if ((R1 < 0.0) && (R2 < 0.0)) return 0.0;
-  if (fabs(R1 - R2) < BARMIN) return 0.0;
-  double flux = 0.0;
-  if ((R1 > R2) && (R1 > BARMIN)) {   // outward
-    if (R2 <= 0.0) {
-      flux = c.nodecode[n1] == 0 ? 0.0
-                                 : -ramp * 0.25 * PI * (diam * diam) * sqrt(2.0 * G * R1 / (1.0 + coef));
-    } else {
-      return c.nodecode[n1] == 0 ? 0.0
-                                 : -ramp * 0.25 * PI * (diam * diam) * sqrt(2.0 * G * (R1 - R2) / coef);
-    }
-  }
-  if ((R2 > R1) && (R2 > BARMIN)) {   // inward
-    if (c.nodecode[n2] == 0) return 0.0;
-    if (R1 <= 0.0) flux = ramp * 0.25 * PI * (diam * diam) * sqrt(2.0 * G * R2 / (1.0 + coef));
-    else flux = ramp * 0.25 * PI * (diam * diam) * sqrt(2.0 * G * (R2 - R1) / coef);
-    c.nib[n1] = 1;
-  }
-  return flux;
-}
-
-__global__ void k_flux_forcing(adc_ctx c, const adc_step_t *steps, const Flags *flags) {
+__global__ void k_flux_forcing(adc_ctx c, const adc_step_t *steps) {
   griddep_wait();
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= c.nvel) return;
-  double *qn0 = c.qn, *qn1 = c.qn + c.nvel, *qn2 = c.qn + 2 * c.nvel;
-  double *en0 = c.en, *en1 = c.en + c.nvel, *en2 = c.en + 2 * c.nvel;
-  qn0[I] = qn1[I];
-  qn1[I] = qn2[I];
-  en0[I] = en1[I];
-  en1[I] = en2[I];
-  double q = 0.0, el = 0.0;
-  const int lb = c.blbc[I];
-  const adc_step_t st = steps[flags->cursor];
-  if (c.flux_on && (lb == 2 || lb == 12 || lb == 22 || lb == 32 || lb == 52)) {
-    const int nf = c.nffr;
-    const size_t nfv = (size_t)nf * c.nvel;
-    const double *famig = c.fconst, *fper = famig + nf, *fff = fper + nf, *fface = fff + nf;
-    const double *qnam = c.fqn, *qnph = c.fqn + nfv, *enam = qnph + nfv, *enph = enam + nfv;
-    const bool coupled = lb == 32 && c.fen;
-    for (int J = 0; J < nf; ++J) {
-      int NCYC = 0;
-      if (fper[J] != 0.0) NCYC = (int)(st.timeh / fper[J]);
-      const double ARGJ = famig[J] * (st.timeh - NCYC * fper[J]) + fface[J];
-      const double RFF = fff[J] * st.rampextflux;
-      q = q + qnam[J + (size_t)nf * I] * RFF * cos(ARGJ - qnph[J + (size_t)nf * I]);
-      if (coupled) el = el + enam[J + (size_t)nf * I] * RFF * cos(ARGJ - enph[J + (size_t)nf * I]);
-    }
-  } else if (c.fser_on) {   // timestep.F:900-902, every entry
-    const SeriesState &ss = c.sstate[1];
-    const size_t r1 = (size_t)ss.k * c.nvel, r2 = r1 + c.nvel;
-    q = st.rampextflux * (c.fser_q[r1 + I] + ss.ratio * (c.fser_q[r2 + I] - c.fser_q[r1 + I]));
-    el = st.rampextflux * (c.fser_e[r1 + I] + ss.ratio * (c.fser_e[r2 + I] - c.fser_e[r1 + I]));
-  }
-  if (lb == 3 || lb == 13 || lb == 23) {
-    // the weir formula with g and BARMIN = 0.04 m (weir_boundary.F90:51);
-    // (RBARWL g)^0.5 as a square root
-    const double RBARWL = 2.0 * (c.eta2[c.bnv[I]] - c.barht[I]) / 3.0;
-    q = RBARWL > 0.04 ? -st.rampintflux * c.barcf[I] * RBARWL * sqrt(RBARWL * c.p.g) : 0.0;
-  }
-  if (lb == 4 || lb == 24 || lb == 5 || lb == 25) q = internal_barrier_flux(c, I, st.rampintflux);
-  if (lb == 5 || lb == 25) q = q + pipe_flux(c, I, st.rampintflux);   // timestep.F:1034-1044
-  qn2[I] = q;
-  en2[I] = el;
-  if (lb == 52) {
-    const int n = c.bnv[I];
-    if (st.it == c.flux_settling_it) {
-      c.etadisc_b[I] = c.eta2[n];
-      c.elevdisc[I] = c.eta2[n];
-    } else if (!flags->etadisc_done && st.it > c.flux_settling_it) {
-      c.elevdisc[I] = c.etadisc_b[I];
-    }
-  }
-  if (lb == 30 || lb == 40 || lb == 41) {
-    const int n = c.bnv[I];
-    const double UN1 = c.uu1[n] * c.bcsii[I] + c.vv1[n] * c.bsiii[I];
-    qn1[I] = c.h2[n] * UN1;
-  }
+  if (I < c.nvel) bnd_forcing(c, steps[c.flags->cursor], I);
 }
 
-// The force of each boundary entry (gwce.F:1783-1815): LBCODEI <= 29 from
-// the specified flux, 30 the radiation condition with the saved H1, 52 the
-// specified flux plus, after FluxSettlingIT, the radiation term.
-__global__ void k_flux_qforce(adc_ctx c, const adc_step_t *steps, Flags *flags) {
+__global__ void k_flux_qforce(adc_ctx c, const adc_step_t *steps) {
   griddep_wait();
   const int J = blockIdx.x * blockDim.x + threadIdx.x;
-  const int it = steps[flags->cursor].it;
+  const int it = steps[c.flags->cursor].it;
   // EtaDisc_Fill ends with the first step at or after FluxSettlingIT; the
   // forcing kernel of this step has read it already
-  if (J == 0 && it >= c.flux_settling_it) flags->etadisc_done = 1;
-  if (J >= c.nvel) return;
-  const double *qn0 = c.qn, *qn1 = c.qn + c.nvel, *qn2 = c.qn + 2 * c.nvel;
-  const int n = c.bnv[J];
-  if (c.blbc[J] == 32) {   // gwce.F:1792-1797
-    const double *en0 = c.en, *en1 = c.en + c.nvel, *en2 = c.en + 2 * c.nvel;
-    const double CELERITY = sqrt(c.p.g * c.h1[n]);
-    const double DT2 = c.p.dt * 2.0;
-    c.qforce[J] = (qn2[J] - qn0[J]) / DT2 - CELERITY * (2.0 * c.etas[n] - (en2[J] - en0[J])) / DT2 +
-                  c.tau0[n] * (qn1[J] - CELERITY * (c.eta1[n] - en1[J]));
-    return;
-  }
-  if (c.blbc[J] == 40 || c.blbc[J] == 41) {   // gwce.F:1804-1805
-    c.qforce[J] = -(qn1[J] - qn0[J]) / c.p.dt - c.tau0[n] * (qn1[J] + qn0[J]) / 2.0;
-    return;
-  }
-  if (c.blbc[J] == 30) {
-    const double CELERITY = sqrt(c.p.g * c.h1[n]);
-    c.qforce[J] = -CELERITY * c.etas[n] / c.p.dt - c.tau0[n] * qn1[J];
-    return;
-  }
-  const double DT2 = c.p.dt * 2.0;
-  double q = (qn2[J] - qn0[J]) / DT2 + c.tau0[n] * qn1[J];
-  if (c.blbc[J] == 52 && it > c.flux_settling_it) {
-    const double Celerity = sqrt(c.p.g * c.h1[n]);
-    q = q - Celerity * (c.etas[n] / c.p.dt + c.tau0[n] * (c.eta1[n] - c.elevdisc[J]));
-  }
-  c.qforce[J] = q;
+  if (J == 0 && it >= c.flux_settling_it) c.flags->etadisc_done = 1;
+  if (J < c.nvel) bnd_qforce(c, it, J);
 }
 
-// One thread per boundary node: its contributions in entry order.
 __global__ void k_flux_rhs(adc_ctx c) {
   griddep_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= c.n_fx) return;
-  const int n = c.fx_node[k];
-  double v = c.gwce_lv[n];
-  for (int q = c.fx_ptr[k]; q < c.fx_ptr[k + 1]; ++q) {
-    const int ent = c.fx_ent[q], j = ent >> 1;
-    const int NCI = c.nodecode[c.bnv[j - 1]], NCJ = c.nodecode[c.bnv[j]];
-    const double B = NCI * NCJ * c.bbl[j - 1] / 4.0;
-    const double qi = c.qforce[j - 1], qj = c.qforce[j];
-    if ((ent & 1) == 0) v = v + B * (2.0 * qi + qj);   // the segment's first node
-    else v = v + B * (2.0 * qj + qi);                  // its second node
-  }
-  c.gwce_lv[n] = v;
+  if (k < c.n_fx) bnd_flux_rhs(c, k);
+}
+
+bool has_flux(const adc_ctx *c) {
+  return c->nfluxf || c->nfluxrbc || c->nfluxgbc || c->nfluxb || c->nfluxib;
 }
 
 int launch_flux_forcing(adc_ctx *c) {
   if (c->eser_on || c->fser_on) {
-    launch_k(k_series_state, 1, 1, c->stream, *c, c->steps, c->flags);
+    launch_k(k_series_state, 1, 1, c->stream, *c, c->steps);
     c->launches++;
   }
-  if (!c->nfluxf && !c->nfluxrbc && !c->nfluxgbc && !c->nfluxb && !c->nfluxib) return ADC_OK;
-  launch_k(k_flux_forcing, nblk(c->nvel), kThreads, c->stream, *c, c->steps, c->flags);
+  if (!has_flux(c)) return ADC_OK;
+  launch_k(k_flux_forcing, nblk(c->nvel), kThreads, c->stream, *c, c->steps);
   c->launches++;
   return ADC_OK;
 }
 
 int launch_flux_rhs(adc_ctx *c) {
-  if (!c->nfluxf && !c->nfluxrbc && !c->nfluxgbc && !c->nfluxb && !c->nfluxib) return ADC_OK;
-  launch_k(k_flux_qforce, nblk(c->nvel), kThreads, c->stream, *c, c->steps, c->flags);
+  if (!has_flux(c)) return ADC_OK;
+  launch_k(k_flux_qforce, nblk(c->nvel), kThreads, c->stream, *c, c->steps);
   launch_k(k_flux_rhs, nblk(c->n_fx), kThreads, c->stream, *c);
   c->launches += 2;
   return ADC_OK;

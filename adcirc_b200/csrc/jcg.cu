@@ -623,7 +623,7 @@ void jcg_clear_barrier(adc_ctx *c) {
   c->launches++;
 }
 
-int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int defer_drift) {
+int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int defer_drift, int d1) {
   JcgArgs a;
   a.do_peror = do_peror;
   a.n = c->np;
@@ -649,7 +649,11 @@ int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int 
   a.arrive = c->jlines;
   a.flags = c->flags;
   a.eta_update = eta_update;
+  a.d1 = d1;
   a.nodecode = c->nodecode;
+  a.nnodecode = c->nnodecode;
+  a.dp = c->dp;
+  a.h0 = c->p.h0;
   a.eta1 = c->eta1;
   a.eta2 = c->eta2;
   a.run_init = run_init;
@@ -678,10 +682,11 @@ int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int 
   return ADC_OK;
 }
 
-// The time-step solve defers the COEF drift to the next GWCE (k_lhs_drift).
-int launch_jcg(adc_ctx *c, int eta_update) {
+// The time-step solve defers the COEF drift to the next GWCE.  `d1` (the
+// resident kernel only): D1 of the wet/dry pass after the elevation update.
+int launch_jcg(adc_ctx *c, int eta_update, bool d1) {
   // a mode with FP32 parts keeps no bitwise COEF history, so the drift is dropped
-  return launch_jcg_impl(c, eta_update, 0, 1, any_f32(c) ? 2 : 1);
+  return launch_jcg_impl(c, eta_update, 0, 1, any_f32(c) ? 2 : 1, d1);
 }
 
 }  // namespace adc

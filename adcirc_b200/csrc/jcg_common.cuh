@@ -26,9 +26,11 @@ struct JcgArgs {
   int defer_drift;            // 1: leave the COEF unscal drift to the next step;
                               // 2: drop it (mixed mode, COEF is rebuilt or kept as is)
   int *drift_pending;         // set to 1 when the drift is left pending
-  const int *nodecode;
-  const double *eta1;
+  int d1;                     // the epilogue ends with wet/dry pass D1 (wetdry.F:234-285)
+  int *nodecode, *nnodecode;
+  const double *eta1, *dp;
   double *eta2;
+  double h0;
   // jcg_ordered.cu: block-local 16-bit columns per slot, rows other blocks read
   const unsigned short *lcol;
   const unsigned char *exp;

@@ -1005,13 +1005,15 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       a.flags->ier = (halt == 2) ? 13 : 0;
       a.flags->zeta = rparm1;
       a.flags->cme = s.con;
+      if (a.d1) a.flags->n_w1_events = 0;
     }
   }
 
-  // ---- epilogue: unscal (itpackv.F:2447-2477) and the GWCE eta update
-  // (gwce.F:2006-2008)
+  // ---- epilogue: unscal (itpackv.F:2447-2477), the GWCE eta update
+  // (gwce.F:2006-2008) and wet/dry pass D1, which took a launch of 2 us and a
+  // second pass over ETA2 and NODECODE by itself
   if (row_warp) {
-    double wv[K], e1[K], uf[K];
+    double wv[K], e1[K], uf[K], dp[K];
     int nc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -1023,6 +1025,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
         if (a.eta_update) {
           e1[k] = a.eta1[i];
           nc[k] = a.nodecode[i];
+          if (a.d1) dp[k] = a.dp[i];
         }
       }
     }
@@ -1034,7 +1037,15 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
         if (a.do_peror) a.u1[i] = uf[k];
         a.u[i] = un;
         a.diag[i] = winv * winv;
-        if (a.eta_update) a.eta2[i] = nc[k] * (un + 0.0) + e1[k];
+        if (a.eta_update) {
+          double e2 = nc[k] * (un + 0.0) + e1[k];
+          if (a.d1 && d1_dries(nc[k], dp[k], a.h0, e2)) {
+            a.nnodecode[i] = 0;
+            a.nodecode[i] = 0;
+            atomicAdd(&a.flags->ncchange, 1);
+          }
+          a.eta2[i] = e2;
+        }
       }
     }
   }

@@ -34,42 +34,29 @@ int cuda_fail(cudaError_t e, const char *what) {
 int jcg_setup_grid(adc_ctx *c, const JcgHostSell *h);
 
 // kernels defined in the other translation units
-__global__ void k_shift_friction(adc_ctx c, const adc_step_t *steps, const Flags *flags);
+__global__ void k_step_begin(adc_ctx c, const adc_step_t *steps, int whole);
 __global__ void k_apply_met(adc_ctx c);
-__global__ void k_lhs_begin(Flags *f, int *words);
-__global__ void k_lhs_drift(adc_ctx c, const int *apply);
-__global__ void k_lhs_drift_flush(int *words);
-template <class R> __global__ void k_lhs_elem(adc_ctx c, const int *rebuild);
-template <class R> __global__ void k_lhs_gather(adc_ctx c, const int *rebuild);
-__global__ void k_lhs_ep(adc_ctx c, const int *rebuild, int nparts);
-__global__ void k_lhs_bc(adc_ctx c, const int *rebuild);
-template <class R> __global__ void k_rhs_elem(adc_ctx c);
-template <class R> __global__ void k_rhs_gather(adc_ctx c);
-__global__ void k_eta_bc(adc_ctx c, const adc_step_t *steps, const Flags *flags);
+__global__ void k_lhs_drift(adc_ctx c);
+__global__ void k_lhs_drift_done(adc_ctx c);
+template <class R> __global__ void k_gwce_elem(adc_ctx c);
+template <class R> __global__ void k_gwce_node(adc_ctx c);
+__global__ void k_gwce_bc(adc_ctx c, const adc_step_t *steps);
 __global__ void k_obc_rhs(adc_ctx c);
-
-__global__ void k_step_end(Flags *f, int *numitr_log, int cap) {
-  griddep_wait();
-  int k = f->cursor;
-  if (k < cap) numitr_log[k] = f->numitr;
-  f->cursor = k + 1;
-}
 
 // Device scratch for the rebuild flag lives after the flags struct.
 static int *rebuild_flag(adc_ctx *c) { return (int *)(c->flags + 1); }
 
-int launch_met_vortex(adc_ctx *c);
 int launch_flux_forcing(adc_ctx *c);
 int launch_flux_rhs(adc_ctx *c);
 int flux_tables(adc_ctx *c, const adc_arrays_t *a);
 int launch_warm_start(adc_ctx *c);
 int launch_predictor_train(adc_ctx *c);
+bool predictor_trains(const adc_ctx *c);
 
-int launch_shift_friction(adc_ctx *c) {
-  launch_k(k_shift_friction, nblk(c->np), kThreads, c->stream, *c, c->steps, c->flags);
+// `whole`: the whole step follows in the same call.
+int launch_shift_friction(adc_ctx *c, bool whole) {
+  launch_k(k_step_begin, nblk(c->np), kThreads, c->stream, *c, c->steps, (int)whole);
   c->launches++;
-  int rc = launch_met_vortex(c);
-  if (rc) return rc;
   if (c->met_pending) {
     launch_k(k_apply_met, nblk(c->np), kThreads, c->stream, *c);
     c->launches++;
@@ -77,75 +64,59 @@ int launch_shift_friction(adc_ctx *c) {
   return launch_flux_forcing(c);   // timestep.F:606-613 and 861-880, after the met forcing
 }
 
-int launch_gwce_lhs(adc_ctx *c) {
-  int *rb = rebuild_flag(c);
-  launch_k(k_lhs_begin, 1, 1, c->stream, c->flags, rb);
-  int nb = nblk(c->np);
-  launch_k(k_lhs_drift, nb, kThreads, c->stream, *c, rb + 2);
+// Matrix and load vector, with their boundary rows.
+int launch_gwce(adc_ctx *c) {
+  const int nbe = nblk(std::max(c->ne, c->np)), nbn = nblk(c->np);
+  // the matrix entries and rows ride in the load vector's spans
   kmark(c, KS_LHS_ELEM, 0);
-  if (f32_assembly(c)) {   // FP32 element assembly
-    launch_k(k_lhs_elem<float>, nblk(c->ne), kThreads, c->stream, *c, rb);
-    kmark(c, KS_LHS_ELEM, 1);
-    kmark(c, KS_LHS_GATHER, 0);
-    launch_k(k_lhs_gather<float>, nb, kThreads, c->stream, *c, rb);
-  } else {
-    launch_k(k_lhs_elem<double>, nblk(c->ne), kThreads, c->stream, *c, rb);
-    kmark(c, KS_LHS_ELEM, 1);
-    kmark(c, KS_LHS_GATHER, 0);
-    launch_k(k_lhs_gather<double>, nb, kThreads, c->stream, *c, rb);
-  }
+  kmark(c, KS_LHS_ELEM, 1);
+  kmark(c, KS_LHS_GATHER, 0);
   kmark(c, KS_LHS_GATHER, 1);
-  launch_k(k_lhs_ep, 1, 1024, c->stream, *c, rb, nb);
-  launch_k(k_lhs_bc, nblk((long long)c->np + c->n_obc), kThreads, c->stream, *c, rb);
-  c->launches += 6;
-  return ADC_OK;
-}
-
-int launch_gwce_rhs(adc_ctx *c) {
   kmark(c, KS_RHS_ELEM, 0);
-  if (f32_assembly(c)) {
-    launch_k(k_rhs_elem<float>, nblk(c->ne), kThreads, c->stream, *c);
+  if (f32_assembly(c)) {   // FP32 element assembly
+    launch_k(k_gwce_elem<float>, nbe, kThreads, c->stream, *c);
     kmark(c, KS_RHS_ELEM, 1);
     kmark(c, KS_RHS_GATHER, 0);
-    launch_k(k_rhs_gather<float>, nblk(c->np), kThreads, c->stream, *c);
+    launch_k(k_gwce_node<float>, nbn, kThreads, c->stream, *c);
   } else {
-    launch_k(k_rhs_elem<double>, nblk(c->ne), kThreads, c->stream, *c);
+    launch_k(k_gwce_elem<double>, nbe, kThreads, c->stream, *c);
     kmark(c, KS_RHS_ELEM, 1);
     kmark(c, KS_RHS_GATHER, 0);
-    launch_k(k_rhs_gather<double>, nblk(c->np), kThreads, c->stream, *c);
+    launch_k(k_gwce_node<double>, nbn, kThreads, c->stream, *c);
   }
   kmark(c, KS_RHS_GATHER, 1);
-  c->launches += 2;
   int rc = launch_flux_rhs(c);   // gwce.F:1737-1834, before the elevation rows
   if (rc) return rc;
-  if (c->neta > 0) {
-    launch_k(k_eta_bc, nblk(c->neta), kThreads, c->stream, *c, c->steps, c->flags);
+  launch_k(k_gwce_bc, nblk((long long)c->np + c->n_obc + c->neta), kThreads, c->stream, *c, c->steps);
+  c->launches += 3;
+  if (c->neta > 0 && c->n_obc_rhs_nodes > 0) {
+    launch_k(k_obc_rhs, nblk(c->n_obc_rhs_nodes), kThreads, c->stream, *c);
     c->launches++;
-    if (c->n_obc_rhs_nodes > 0) {
-      launch_k(k_obc_rhs, nblk(c->n_obc_rhs_nodes), kThreads, c->stream, *c);
-      c->launches++;
-    }
   }
   return ADC_OK;
 }
 
-// The whole 2DDI step (TIMESTEP order), without host synchronisation.
-static int enqueue_step(adc_ctx *c, bool timed) {
+// The whole 2DDI step (TIMESTEP order), without host synchronisation.  With
+// `log`, a step of adc_run: its iteration count goes there, and the step
+// table's cursor advances.
+static int enqueue_step(adc_ctx *c, bool timed, int *log) {
   int rc;
   c->kmark = timed ? 1 : 0;
   if (timed) cudaEventRecordWithFlags(c->ev[0], c->stream, cudaEventRecordExternal);
-  if ((rc = launch_shift_friction(c))) return rc;
+  if ((rc = launch_shift_friction(c, true))) return rc;
   if (timed) cudaEventRecordWithFlags(c->ev[1], c->stream, cudaEventRecordExternal);
-  if ((rc = launch_gwce_lhs(c))) return rc;
-  if ((rc = launch_gwce_rhs(c))) return rc;
+  if ((rc = launch_gwce(c))) return rc;
   if ((rc = launch_warm_start(c))) return rc;
   if (timed) cudaEventRecordWithFlags(c->ev[2], c->stream, cudaEventRecordExternal);
-  if ((rc = launch_jcg(c, 1))) return rc;
+  // D1 of the wet/dry pass ends the resident solve, unless the predictor's
+  // training reads the solution first
+  const bool d1 = c->p.nolifa == 2 && (c->jcg_res == 1 || c->jcg_res == 2) && !predictor_trains(c);
+  if ((rc = launch_jcg(c, 1, d1))) return rc;
   if ((rc = launch_predictor_train(c))) return rc;   // nothing unless training is on
   if (timed) cudaEventRecordWithFlags(c->ev[3], c->stream, cudaEventRecordExternal);
-  if ((rc = launch_wetdry(c))) return rc;
+  if ((rc = launch_wetdry(c, true, d1))) return rc;
   if (timed) cudaEventRecordWithFlags(c->ev[4], c->stream, cudaEventRecordExternal);
-  if ((rc = launch_momentum(c))) return rc;
+  if ((rc = launch_momentum(c, true, log))) return rc;
   if (timed) cudaEventRecordWithFlags(c->ev[5], c->stream, cudaEventRecordExternal);
   c->kmark = 0;
   return ADC_OK;
@@ -423,9 +394,8 @@ static int download_state(adc_ctx *c) {
   TRY(down(a->mju, c->mju, np));
   if (a->coef) {
     // COEF as the reference holds it: apply a drift the last solve left pending
-    int *w = rebuild_flag(c);
-    launch_k(k_lhs_drift_flush, 1, 1, c->stream, w);
-    launch_k(k_lhs_drift, nblk(np), kThreads, c->stream, *c, w + 2);
+    launch_k(k_lhs_drift, nblk(np), kThreads, c->stream, *c);
+    launch_k(k_lhs_drift_done, 1, 1, c->stream, *c);
     ADC_CUDA(cudaGetLastError());
     ADC_CUDA(cudaStreamSynchronize(c->stream));
     std::vector<double> d(np), o(std::max(c->nnz_pad, 1));
@@ -659,6 +629,7 @@ static int bind_impl(const adc_params_t *p, const adc_arrays_t *a, int prec, adc
     char *f = nullptr;
     if (cudaMalloc((void **)&f, sizeof(Flags) + 64) != cudaSuccess) return fail(ADC_ERR_NOMEM);
     c->flags = (Flags *)f;
+    c->tickets = (int *)(c->flags + 1) + 4;   // after the four LHS words
   }
   c->steps_cap = 1;
   B(dalloc(&c->steps, 1));
@@ -677,8 +648,8 @@ static int bind_impl(const adc_params_t *p, const adc_arrays_t *a, int prec, adc
   memset(&fl, 0, sizeof(fl));
   fl.ncchange = 1;   // adcirc.F:404: the matrix is built on the first step
   B(up(c->flags, &fl, 1));
-  int words[4] = {0, 0, 0, 1};   // rebuild, drift pending/apply, gather every row
-  B(up(rebuild_flag(c), words, 4));
+  int words[6] = {0, 0, 0, 1, 0, 0};   // rebuild, drift pending/applied, gather every row, tickets
+  B(up(rebuild_flag(c), words, 6));
   ADC_CUDA(cudaDeviceSynchronize());
 #undef B
   *out = c;
@@ -719,14 +690,14 @@ static int set_single_step(adc_ctx *c, const adc_step_t *s) {
 // graph of the step (phase events included), so the per-step call pays no
 // per-kernel launch cost.
 static int run_single_step(adc_ctx *c) {
-  if (c->met_pending) return enqueue_step(c, true);
+  if (c->met_pending) return enqueue_step(c, true, nullptr);
   if (!c->graph1_ok) {
     cudaGraph_t g = nullptr;
     int64_t l0 = c->launches;
     cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
     int rc = ADC_OK;
     if (e == cudaSuccess) {
-      rc = enqueue_step(c, true);
+      rc = enqueue_step(c, true, nullptr);
       cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
       if (e2 != cudaSuccess) e = e2;
     }
@@ -741,7 +712,7 @@ static int run_single_step(adc_ctx *c) {
       fprintf(stderr, "adcgpu: single-step graph not used (%s, rc %d)\n", cudaGetErrorString(e), rc);
     cudaGetLastError();
   }
-  if (!c->graph1_ok) return enqueue_step(c, true);
+  if (!c->graph1_ok) return enqueue_step(c, true, nullptr);
   ADC_CUDA(cudaGraphLaunch(c->graph1, c->stream));
   c->launches += c->graph1_launches;
   return ADC_OK;
@@ -769,7 +740,7 @@ int adc_gpu_free(adc_ctx *c) {
 int adc_shift_friction(adc_ctx *c, const adc_step_t *s) {
   if (!c) return ADC_ERR_ARG;
   TRY(set_single_step(c, s));
-  TRY(launch_shift_friction(c));
+  TRY(launch_shift_friction(c, false));
   c->met_pending = 0;
   ADC_CUDA(cudaGetLastError());
   ADC_CUDA(cudaStreamSynchronize(c->stream));
@@ -779,10 +750,9 @@ int adc_shift_friction(adc_ctx *c, const adc_step_t *s) {
 int adc_gwce_new(adc_ctx *c, const adc_step_t *s, adc_stepout_t *out) {
   if (!c) return ADC_ERR_ARG;
   TRY(set_single_step(c, s));
-  TRY(launch_gwce_lhs(c));
-  TRY(launch_gwce_rhs(c));
+  TRY(launch_gwce(c));
   TRY(launch_warm_start(c));
-  TRY(launch_jcg(c, 1));
+  TRY(launch_jcg(c, 1, false));
   TRY(launch_predictor_train(c));
   ADC_CUDA(cudaGetLastError());
   Flags f;
@@ -794,7 +764,7 @@ int adc_gwce_new(adc_ctx *c, const adc_step_t *s, adc_stepout_t *out) {
 int adc_wetdry(adc_ctx *c, const adc_step_t *s, adc_stepout_t *out) {
   if (!c) return ADC_ERR_ARG;
   TRY(set_single_step(c, s));
-  TRY(launch_wetdry(c));
+  TRY(launch_wetdry(c, false, false));
   ADC_CUDA(cudaGetLastError());
   Flags f;
   TRY(read_flags(c, f));
@@ -805,7 +775,7 @@ int adc_wetdry(adc_ctx *c, const adc_step_t *s, adc_stepout_t *out) {
 int adc_momentum(adc_ctx *c, const adc_step_t *s) {
   if (!c) return ADC_ERR_ARG;
   TRY(set_single_step(c, s));
-  TRY(launch_momentum(c));
+  TRY(launch_momentum(c, false, nullptr));
   ADC_CUDA(cudaGetLastError());
   ADC_CUDA(cudaStreamSynchronize(c->stream));
   return ADC_OK;
@@ -850,11 +820,10 @@ int adc_run(adc_ctx *c, int nsteps, const adc_step_t *steps, int *numitr, adc_st
     cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
     int rc = ADC_OK;
     if (e == cudaSuccess) {
-      rc = enqueue_step(c, false);
-      launch_k(k_step_end, 1, 1, c->stream, c->flags, c->numitr_log, c->numitr_cap);
+      rc = enqueue_step(c, false, c->numitr_log);
       e = cudaStreamEndCapture(c->stream, &g);
     }
-    c->graph_launches = (int)(c->launches - l0) + 1;
+    c->graph_launches = (int)(c->launches - l0);
     c->launches = l0;
     if (e == cudaSuccess && rc == ADC_OK) {
       e = cudaGraphInstantiate(&c->graph, g, 0);
@@ -869,9 +838,7 @@ int adc_run(adc_ctx *c, int nsteps, const adc_step_t *steps, int *numitr, adc_st
       ADC_CUDA(cudaGraphLaunch(c->graph, c->stream));
       c->launches += c->graph_launches;
     } else {
-      TRY(enqueue_step(c, false));
-      launch_k(k_step_end, 1, 1, c->stream, c->flags, c->numitr_log, c->numitr_cap);
-      c->launches++;
+      TRY(enqueue_step(c, false, c->numitr_log));
     }
   }
   ADC_CUDA(cudaEventRecord(c->run_ev[1], c->stream));
@@ -1033,9 +1000,8 @@ static int ens_capture(adc_ensemble *e) {
     adc_ctx *c = e->m[k];
     cudaStreamWaitEvent(c->stream, e->fork, 0);
     int64_t l0 = c->launches;
-    rc = enqueue_step(c, false);
-    launch_k(k_step_end, 1, 1, c->stream, c->flags, c->numitr_log, c->numitr_cap);
-    c->graph_launches = (int)(c->launches - l0) + 1;
+    rc = enqueue_step(c, false, c->numitr_log);
+    c->graph_launches = (int)(c->launches - l0);
     c->launches = l0;
     cudaEventRecord(e->join[k], c->stream);
     cudaStreamWaitEvent(e->root, e->join[k], 0);
