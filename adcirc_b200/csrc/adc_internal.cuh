@@ -118,8 +118,9 @@ struct adc_ctx {
   // matrix structure (SELL)
   int *sl_ptr, *sl_w, *col, *rlen;
   int *lhs_src;          // 2 per padded slot: index 6*e+q of the element off-diagonal value, or -1
-  int *ell_of_sell;      // host-side sync helper: SELL slot -> (i + np*j) ELL index (device copy unused)
-  int *h_ell_of_sell;
+  int *h_ell_of_sell;    // host: SELL slot -> (i + np*j) index into COEF, -1 for padding
+  unsigned long long *h_pack;   // pinned block the state goes through (sync.cu), null if it is large
+  size_t pack_half;             // words of one of its halves
   // boundaries
   int *nbd, *is_nbd;     // is_nbd[i] = I index (0-based) or -1
   double *amig, *per, *face, *ff, *emo, *efa;

@@ -36,8 +36,6 @@ int jcg_setup_grid(adc_ctx *c, const JcgHostSell *h);
 // kernels defined in the other translation units
 __global__ void k_step_begin(adc_ctx c, const adc_step_t *steps, int whole);
 __global__ void k_apply_met(adc_ctx c);
-__global__ void k_lhs_drift(adc_ctx c);
-__global__ void k_lhs_drift_done(adc_ctx c);
 template <class R> __global__ void k_gwce_elem(adc_ctx c);
 template <class R> __global__ void k_gwce_node(adc_ctx c);
 __global__ void k_gwce_bc(adc_ctx c, const adc_step_t *steps);
@@ -46,6 +44,8 @@ __global__ void k_obc_rhs(adc_ctx c);
 // Device scratch for the rebuild flag lives after the flags struct.
 static int *rebuild_flag(adc_ctx *c) { return (int *)(c->flags + 1); }
 
+void sync_setup(adc_ctx *c);
+int download_state(adc_ctx *c);
 int launch_flux_forcing(adc_ctx *c);
 int launch_flux_rhs(adc_ctx *c);
 int flux_tables(adc_ctx *c, const adc_arrays_t *a);
@@ -137,13 +137,6 @@ template <class T>
 static int up(T *d, const T *h, size_t n) {
   if (n == 0) return ADC_OK;
   ADC_CUDA(cudaMemcpy(d, h, n * sizeof(T), cudaMemcpyHostToDevice));
-  return ADC_OK;
-}
-
-template <class T>
-static int down(T *h, const T *d, size_t n) {
-  if (n == 0 || h == nullptr) return ADC_OK;
-  ADC_CUDA(cudaMemcpy(h, d, n * sizeof(T), cudaMemcpyDeviceToHost));
   return ADC_OK;
 }
 
@@ -358,58 +351,6 @@ static int upload_state(adc_ctx *c) {
   return ADC_OK;
 }
 
-static int download_state(adc_ctx *c) {
-  adc_arrays_t *a = &c->host;
-  const int np = c->np, ne = c->ne;
-  ADC_CUDA(cudaStreamSynchronize(c->stream));
-  TRY(down(a->eta1, c->eta1, np));
-  TRY(down(a->eta2, c->eta2, np));
-  TRY(down(a->etas, c->etas, np));
-  TRY(down(a->uu1, c->uu1, np));
-  TRY(down(a->vv1, c->vv1, np));
-  TRY(down(a->uu2, c->uu2, np));
-  TRY(down(a->vv2, c->vv2, np));
-  TRY(down(a->qx1, c->qx1, np));
-  TRY(down(a->qy1, c->qy1, np));
-  TRY(down(a->qx2, c->qx2, np));
-  TRY(down(a->qy2, c->qy2, np));
-  TRY(down(a->h1, c->h1, np));
-  TRY(down(a->h2, c->h2, np));
-  TRY(down(a->tk, c->tk, np));
-  TRY(down(a->tkm, c->tkm, 3 * (size_t)np));
-  TRY(down(a->totalarea, c->totalarea, np));
-  TRY(down(a->alphal, c->alphal, ne));
-  TRY(down(a->wsx1, c->wsx1, np));
-  TRY(down(a->wsy1, c->wsy1, np));
-  TRY(down(a->wsx2, c->wsx2, np));
-  TRY(down(a->wsy2, c->wsy2, np));
-  TRY(down(a->pr1, c->pr1, np));
-  TRY(down(a->pr2, c->pr2, np));
-  TRY(down(a->gwce_lv, c->gwce_lv, np));
-  TRY(down(a->mom_lv_x, c->mom_x, np));
-  TRY(down(a->mom_lv_y, c->mom_y, np));
-  TRY(down(a->nodecode, c->nodecode, np));
-  TRY(down(a->nnodecode, c->nnodecode, np));
-  TRY(down(a->noff, c->noff, ne));
-  TRY(down(a->mju, c->mju, np));
-  if (a->coef) {
-    // COEF as the reference holds it: apply a drift the last solve left pending
-    launch_k(k_lhs_drift, nblk(np), kThreads, c->stream, *c);
-    launch_k(k_lhs_drift_done, 1, 1, c->stream, *c);
-    ADC_CUDA(cudaGetLastError());
-    ADC_CUDA(cudaStreamSynchronize(c->stream));
-    std::vector<double> d(np), o(std::max(c->nnz_pad, 1));
-    TRY(down(d.data(), c->diag, np));
-    TRY(down(o.data(), c->offd, c->nnz_pad));
-    std::fill(a->coef, a->coef + (size_t)np * c->mnei, 0.0);
-    for (int i = 0; i < np; ++i) a->coef[i] = d[i];
-    for (int idx = 0; idx < c->nnz_pad; ++idx)
-      if (c->h_ell_of_sell[idx] >= 0) a->coef[c->h_ell_of_sell[idx]] = o[idx];
-  }
-  TRY(down(a->obccoef, c->obccoef, (size_t)c->neta * (c->mnei - 1)));
-  return ADC_OK;
-}
-
 void mp_free(adc_ctx *c);
 
 static void free_ctx(adc_ctx *c) {
@@ -463,6 +404,7 @@ static void free_ctx(adc_ctx *c) {
     if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete[] c->h_ell_of_sell;
+  if (c->h_pack) cudaFreeHost(c->h_pack);
   delete c;
 }
 
@@ -636,6 +578,7 @@ static int bind_impl(const adc_params_t *p, const adc_arrays_t *a, int prec, adc
   c->numitr_cap = 1;
   B(dalloc(&c->numitr_log, 1));
   B(upload_state(c));
+  sync_setup(c);
   Itp itp;
   memset(&itp, 0, sizeof(itp));
   itp.rparm1 = p->convcr;
