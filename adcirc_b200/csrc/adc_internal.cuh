@@ -209,6 +209,8 @@ struct adc_ctx {
   size_t jcg_smem;
   int jcg_stage_wcap;
   unsigned char *jtab;         // one allocation behind the tables below
+  unsigned char *jtab_room;    // the caller's room for them, if it has any
+  size_t jtab_cap;
   unsigned short *jlcol;
   uint4 *jrcol;
   int4 *jmeta;

@@ -14,6 +14,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 #include <algorithm>
 
@@ -26,23 +27,48 @@ static int g_q1 = 0;
 int jcg_q1_get() { return g_q1; }
 void jcg_q1_set(int v) { g_q1 = v; }
 
+// One call's device memory: one allocation.  (A cudaMalloc takes 1 to 3 ms
+// for each block of a megabyte or more, and so does its cudaFree; the 18
+// arrays of a 90k-row system were 20 to 70 ms around a solve of 0.12 ms.)
 struct Stage {
   adc_ctx c;
+  unsigned char *base = nullptr;
+  size_t used = 0;
   Stage() { memset((void *)&c, 0, sizeof(c)); }
   ~Stage() {
-    void *ptrs[] = {c.sl_ptr, c.sl_w, c.col, c.rlen, c.offd, c.soff, c.diag, c.gwce_lv, c.etas, c.ju1,
-                    c.jp[0], c.jp[1], c.jw, c.jtab, c.itp, c.bar, c.flags, c.jlines};
-    for (void *p : ptrs)
-      if (p) cudaFree(p);
-    if (c.stream) cudaStreamDestroy(c.stream);
+    if (c.stream) {
+      cudaStreamSynchronize(c.stream);   // copies from this call's host arrays
+      cudaStreamDestroy(c.stream);
+    }
+    if (c.jtab && c.jtab != c.jtab_room) cudaFree(c.jtab);
+    if (base) cudaFree(base);
+  }
+  // Places `n` elements: first for the size alone, then in the allocation.
+  template <class T>
+  void place(T **d, size_t n) {
+    used = (used + 255) & ~(size_t)255;
+    if (base) *d = (T *)(base + used);
+    used += std::max<size_t>(n, 1) * sizeof(T);
   }
 };
 
-template <class T>
-static cudaError_t alloc_up(T **d, const T *h, size_t n) {
-  cudaError_t e = cudaMalloc((void **)d, std::max<size_t>(n, 1) * sizeof(T));
-  if (e != cudaSuccess || !h || n == 0) return e;
-  return cudaMemcpy(*d, h, n * sizeof(T), cudaMemcpyHostToDevice);
+// The scalars a solve reads and leaves, copied together.
+struct SolveState {
+  Itp it;
+  Bar bar;
+  Flags fl;
+};
+
+// SELL slots from COEF as the caller holds it (columns of n rows), and back.
+__global__ void k_slots_from_ell(int nnz, const int *src, const double *ell, double *off) {
+  griddep_wait();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < nnz) off[t] = src[t] >= 0 ? ell[src[t]] : 0.0;
+}
+__global__ void k_slots_to_ell(int nnz, const int *src, const double *off, double *ell) {
+  griddep_wait();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < nnz && src[t] >= 0) ell[src[t]] = off[t];
 }
 
 static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, double *rhs,
@@ -51,35 +77,39 @@ static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, doubl
   // sliced ELL of the slots that take part in pjac: every j >= 2 except the
   // empty ones (jcoef == i and coef == 0, i.e. 0*u(i) terms)
   const int nslices = (n + kSlice - 1) / kSlice;
-  std::vector<int> rlen(n, 0), sl_w(nslices, 0), sl_ptr(nslices + 1, 0);
-  std::vector<std::vector<int>> rows(n);
-  for (int i = 0; i < n; ++i) {
-    for (int j = 1; j < maxnz; ++j) {
-      size_t k = i + (size_t)ndim * j;
-      if (jcoef[k] == i + 1 && coef[k] == 0.0) continue;
-      rows[i].push_back(j);
-    }
-    rlen[i] = (int)rows[i].size();
-    sl_w[i / kSlice] = std::max(sl_w[i / kSlice], rlen[i]);
+  const size_t npad = (size_t)nslices * kSlice;
+  std::vector<int> rlen(npad, 0), sl_w(nslices, 0), sl_ptr(nslices + 1, 0);
+  for (int j = 1; j < maxnz; ++j) {
+    const int *jc = jcoef + (size_t)ndim * j;
+    const double *cf = coef + (size_t)ndim * j;
+    for (int i = 0; i < n; ++i) rlen[i] += !(jc[i] == i + 1 && cf[i] == 0.0);
   }
-  for (int s = 0; s < nslices; ++s) sl_ptr[s + 1] = sl_ptr[s] + sl_w[s] * kSlice;
+  for (int i = 0; i < n; ++i) sl_w[i / kSlice] = std::max(sl_w[i / kSlice], rlen[i]);
+  size_t rcol = 0;
+  for (int s = 0; s < nslices; ++s) {
+    sl_ptr[s + 1] = sl_ptr[s] + sl_w[s] * kSlice;
+    rcol += 512 * ((sl_w[s] + 7) / 8);
+  }
   const int nnz = sl_ptr[nslices];
-  std::vector<int> col(std::max(nnz, 1), 0), src(std::max(nnz, 1), -1);
-  std::vector<double> off(std::max(nnz, 1), 0.0), diag(n);
-  for (int i = 0; i < n; ++i) {
-    diag[i] = coef[i];
-    int s = i / kSlice, lane = i % kSlice;
-    for (int k = 0; k < sl_w[s]; ++k) {
-      int idx = sl_ptr[s] + k * kSlice + lane;
-      if (k < rlen[i]) {
-        size_t e = i + (size_t)ndim * rows[i][k];
-        col[idx] = jcoef[e] - 1;
-        off[idx] = coef[e];
-        src[idx] = (int)e;
-      } else {
-        col[idx] = i;
+  // column and source of each slot; both arrays are written in full
+  const std::unique_ptr<int[]> col(new int[std::max(nnz, 1)]), src(new int[std::max(nnz, 1)]);
+  for (int s = 0; s < nslices; ++s) {
+    int at[kSlice] = {0};
+    const int i0 = s * kSlice, lanes = std::min(kSlice, n - i0);
+    int *cs = col.get() + sl_ptr[s], *ss = src.get() + sl_ptr[s];
+    for (int j = 1; j < maxnz; ++j)
+      for (int l = 0; l < lanes; ++l) {
+        const size_t k = i0 + l + (size_t)ndim * j;
+        if (jcoef[k] == i0 + l + 1 && coef[k] == 0.0) continue;
+        const int q = at[l]++ * kSlice + l;
+        cs[q] = jcoef[k] - 1;
+        ss[q] = i0 + l + n * j;
       }
-    }
+    for (int l = 0; l < kSlice; ++l)
+      for (int q = at[l] * kSlice + l; q < sl_w[s] * kSlice; q += kSlice) {
+        cs[q] = l < lanes ? i0 + l : 0;
+        ss[q] = -1;
+      }
   }
   Stage st;
   adc_ctx &c = st.c;
@@ -88,35 +118,67 @@ static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, doubl
   c.nnz_pad = nnz;
   c.itmax = itmax;
   if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess) return ADC_ERR_CUDA;
-  ADC_CUDA(alloc_up(&c.sl_ptr, sl_ptr.data(), sl_ptr.size()));
-  ADC_CUDA(alloc_up(&c.sl_w, sl_w.data(), sl_w.size()));
-  ADC_CUDA(alloc_up(&c.col, col.data(), col.size()));
-  rlen.resize((size_t)nslices * kSlice, 0);
-  ADC_CUDA(alloc_up(&c.rlen, rlen.data(), rlen.size()));
-  ADC_CUDA(alloc_up(&c.offd, off.data(), off.size()));
-  ADC_CUDA(alloc_up<double>(&c.soff, nullptr, off.size()));
-  ADC_CUDA(alloc_up(&c.diag, diag.data(), n));
-  ADC_CUDA(alloc_up(&c.gwce_lv, rhs, n));
-  const size_t npad = (size_t)nslices * kSlice;
-  ADC_CUDA(alloc_up<double>(&c.etas, nullptr, npad));
-  ADC_CUDA(cudaMemset(c.etas, 0, npad * sizeof(double)));
-  ADC_CUDA(cudaMemcpy(c.etas, u, n * sizeof(double), cudaMemcpyHostToDevice));
-  double **vec[] = {&c.ju1, &c.jw};
-  for (double **v : vec) {
-    ADC_CUDA(alloc_up<double>(v, nullptr, npad));
-    ADC_CUDA(cudaMemset(*v, 0, npad * sizeof(double)));
+  double *d_ell = nullptr;
+  int *d_src = nullptr;
+  SolveState *d_state = nullptr;
+  // room for the solver's tables: packed columns, and at most every slot a
+  // halo node that some block sends
+  const size_t room = rcol + 14 * (size_t)nnz + 4 * npad + (64u << 10);
+  const size_t nlines = 2 * 128 * 1024;   // of up to 1,024 row blocks (two per SM at most)
+  size_t zero0 = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    if (pass == 1) ADC_CUDA(cudaMalloc((void **)&st.base, st.used));
+    st.used = 0;
+    st.place(&c.sl_ptr, nslices + 1);
+    st.place(&c.sl_w, nslices);
+    st.place(&c.col, nnz);
+    st.place(&c.rlen, npad);
+    st.place(&c.offd, nnz);
+    st.place(&c.soff, nnz);
+    st.place(&c.diag, n);
+    st.place(&c.gwce_lv, n);
+    st.place(&d_ell, (size_t)n * maxnz);
+    st.place(&d_src, nnz);
+    st.place(&d_state, 1);
+    st.place(&c.jtab_room, room);
+    st.place((char **)&c.jlines, nlines);
+    zero0 = (st.used + 255) & ~(size_t)255;   // from here on zeroed
+    st.place(&c.etas, npad);
+    st.place(&c.ju1, npad);
+    st.place(&c.jw, npad);
+    st.place(&c.jp[0], npad);
+    st.place(&c.jp[1], npad);
   }
-  ADC_CUDA(alloc_up<double4>(&c.jp[0], nullptr, npad));
-  ADC_CUDA(alloc_up<double4>(&c.jp[1], nullptr, npad));
-  ADC_CUDA(cudaMemset(c.jp[0], 0, npad * sizeof(double4)));
-  ADC_CUDA(cudaMemset(c.jp[1], 0, npad * sizeof(double4)));
-  const JcgHostSell hs{sl_ptr.data(), sl_w.data(), col.data(), rlen.data()};
+  c.jtab_cap = room;
+  c.itp = &d_state->it;
+  c.bar = &d_state->bar;
+  c.flags = &d_state->fl;
+  // everything in stream order (pageable copies may still be on their way
+  // when the call returns)
+  auto up = [&](void *d, const void *h, size_t bytes) {
+    return bytes ? cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c.stream) : cudaSuccess;
+  };
+  ADC_CUDA(cudaMemsetAsync(st.base + zero0, 0, st.used - zero0, c.stream));
+  ADC_CUDA(up(c.sl_ptr, sl_ptr.data(), sl_ptr.size() * sizeof(int)));
+  ADC_CUDA(up(c.sl_w, sl_w.data(), sl_w.size() * sizeof(int)));
+  ADC_CUDA(up(c.col, col.get(), (size_t)nnz * sizeof(int)));
+  ADC_CUDA(up(c.rlen, rlen.data(), rlen.size() * sizeof(int)));
+  ADC_CUDA(up(d_src, src.get(), (size_t)nnz * sizeof(int)));
+  ADC_CUDA(up(c.diag, coef, n * sizeof(double)));
+  ADC_CUDA(up(c.gwce_lv, rhs, n * sizeof(double)));
+  ADC_CUDA(up(c.etas, u, n * sizeof(double)));
+  ADC_CUDA(cudaMemcpy2DAsync(d_ell, n * sizeof(double), coef, (size_t)ndim * sizeof(double), n * sizeof(double),
+                             maxnz, cudaMemcpyHostToDevice, c.stream));
+  launch_k(k_slots_from_ell, std::max(1, nblk(nnz)), kThreads, c.stream, nnz, (const int *)d_src,
+           (const double *)d_ell, c.offd);
+  const JcgHostSell hs{sl_ptr.data(), sl_w.data(), col.get(), rlen.data()};
   int rc = jcg_setup_grid(&c, &hs);
   if (rc) return rc;
-  ADC_CUDA(alloc_up<char>((char **)&c.jlines, nullptr, 2 * 128 * (size_t)c.jcg_rows_blocks));
+  if (2 * 128 * (size_t)c.jcg_rows_blocks > nlines) { set_error("JCG barrier lines"); return ADC_ERR_ARG; }
   jcg_clear_barrier(&c);
-  Itp it;
-  memset(&it, 0, sizeof(it));
+  SolveState ss;
+  memset((void *)&ss, 0, sizeof(ss));
+  Itp &it = ss.it;
   it.zeta = rparm[0];
   it.rparm1 = rparm[0];
   it.cme = rparm[1];
@@ -128,25 +190,25 @@ static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, doubl
   double temp = 512.0 * DBL_EPSILON;
   if (it.zeta < temp) it.zeta = temp;
   it.rec.need_unorm = !it.q1;
-  ADC_CUDA(alloc_up(&c.itp, &it, 1));
-  Bar bar = {0, 0};
-  ADC_CUDA(alloc_up(&c.bar, &bar, 1));
-  Flags fl;
-  memset(&fl, 0, sizeof(fl));
-  ADC_CUDA(alloc_up(&c.flags, &fl, 1));
+  ADC_CUDA(up(d_state, &ss, sizeof(ss)));
   rc = launch_jcg_impl(&c, 0, iparm[11] >= 0 ? 1 : 0, 0, 0, 0);
   if (rc) return rc;
+  launch_k(k_slots_to_ell, std::max(1, nblk(nnz)), kThreads, c.stream, nnz, (const int *)d_src,
+           (const double *)c.offd, d_ell);
+  ADC_CUDA(cudaMemcpyAsync(&ss, d_state, sizeof(ss), cudaMemcpyDeviceToHost, c.stream));
   ADC_CUDA(cudaStreamSynchronize(c.stream));
-  ADC_CUDA(cudaMemcpy(&fl, c.flags, sizeof(fl), cudaMemcpyDeviceToHost));
+  const Flags &fl = ss.fl;
   if (fl.timeout) { set_error("JCG barrier wait expired"); return ADC_ERR_TIMEOUT; }
-  ADC_CUDA(cudaMemcpy(&it, c.itp, sizeof(it), cudaMemcpyDeviceToHost));
-  ADC_CUDA(cudaMemcpy(u, c.etas, n * sizeof(double), cudaMemcpyDeviceToHost));
-  ADC_CUDA(cudaMemcpy(rhs, c.gwce_lv, n * sizeof(double), cudaMemcpyDeviceToHost));
-  ADC_CUDA(cudaMemcpy(diag.data(), c.diag, n * sizeof(double), cudaMemcpyDeviceToHost));
-  ADC_CUDA(cudaMemcpy(off.data(), c.offd, nnz * sizeof(double), cudaMemcpyDeviceToHost));
-  for (int i = 0; i < n; ++i) coef[i] = diag[i];
-  for (int idx = 0; idx < nnz; ++idx)
-    if (src[idx] >= 0) coef[src[idx]] = off[idx];
+  auto down = [&](void *h, const void *d, size_t bytes) {
+    return cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c.stream);
+  };
+  ADC_CUDA(down(u, c.etas, n * sizeof(double)));
+  ADC_CUDA(down(rhs, c.gwce_lv, n * sizeof(double)));
+  ADC_CUDA(down(coef, c.diag, n * sizeof(double)));
+  if (maxnz > 1)
+    ADC_CUDA(cudaMemcpy2DAsync(coef + ndim, (size_t)ndim * sizeof(double), d_ell + n, n * sizeof(double),
+                               n * sizeof(double), maxnz - 1, cudaMemcpyDeviceToHost, c.stream));
+  ADC_CUDA(cudaStreamSynchronize(c.stream));
   g_q1 = it.q1;
   ier = fl.ier;
   in_out = it.in;

@@ -67,8 +67,10 @@ struct JcgTables {
     return o;
   }
   int upload(adc_ctx *c) const {
-    ADC_CUDA(cudaMalloc((void **)&c->jtab, h.size() + 256));
-    ADC_CUDA(cudaMemcpy(c->jtab, h.data(), h.size(), cudaMemcpyHostToDevice));
+    if (h.size() + 256 <= c->jtab_cap) c->jtab = c->jtab_room;
+    else ADC_CUDA(cudaMalloc((void **)&c->jtab, h.size() + 256));
+    ADC_CUDA(cudaMemcpyAsync(c->jtab, h.data(), h.size(), cudaMemcpyHostToDevice, c->stream));
+    ADC_CUDA(cudaStreamSynchronize(c->stream));
     return ADC_OK;
   }
 };

@@ -90,3 +90,40 @@ def test_layouts(n, wide, huge):
         assert np.abs(r - r2).max() <= REL_TOL * np.abs(r2).max()
     assert np.array_equal(jg, jo)
     assert np.abs(cg - co).max() <= 1e-14 * np.abs(co).max()
+
+
+@pytest.mark.parametrize("n,pad", [(1, 3), (33, 1), (500, 7), (20_001, 31)])
+def test_padded_columns(n, pad):
+    """COEF with NDIM > N and a column of empty slots: the solution, the
+    drifted COEF and its untouched parts as the oracle leaves them (COEF to
+    1e-13, as in the other drop-in tests)."""
+    import oracle
+    from adcirc_b200 import _lib
+    lib, orc = _lib.load(), oracle.load()
+    from adcirc_b200._lib import dp_, ip_, ptr
+    maxnz, jc, cf, rhs, u0 = _system(n, n + 1)
+    ndim, maxnz = n + pad, maxnz + 1
+    jcoef = np.full((ndim, maxnz), 9, np.int32, order="F")
+    coef = np.full((ndim, maxnz), 7.5, order="F")
+    jcoef[:n], coef[:n] = 0, 0.0
+    jcoef[:n, :-1], coef[:n, :-1] = jc, cf
+    got = []
+    for jcg, dfault, reset in ((lib.adc_jcg, lib.adc_dfault, lib.adc_jcg_reset),
+                               (orc.orc_jcg, orc.orc_dfault, orc.orc_itpack_reset)):
+        reset()
+        j, c, r, u = jcoef.copy(order="F"), coef.copy(order="F"), rhs.copy(), u0.copy()
+        iparm, rparm = np.zeros(12, np.int32), np.zeros(12)
+        dfault(ptr(iparm, ip_), ptr(rparm, dp_))
+        iparm[0], rparm[0] = 200, 1e-10
+        nw = 4 * n + 4 * 200
+        wksp, iwksp, ier = np.zeros(nw + 16), np.zeros(3 * n, np.int32), C.c_int(-1)
+        jcg(C.byref(C.c_int(n)), C.byref(C.c_int(ndim)), C.byref(C.c_int(maxnz)), ptr(j, ip_), ptr(c, dp_),
+            ptr(r, dp_), ptr(u, dp_), ptr(iwksp, ip_), C.byref(C.c_int(nw)), ptr(wksp, dp_),
+            ptr(iparm, ip_), ptr(rparm, dp_), C.byref(ier))
+        got.append((ier.value, iparm[0], j, c, r, u))
+    g, o = got
+    assert g[:2] == o[:2]
+    assert np.array_equal(g[2], o[2]) and np.array_equal(g[3][n:], coef[n:])
+    assert np.abs(g[3] - o[3]).max() <= 1e-13 * np.abs(o[3]).max()
+    assert np.abs(g[4] - o[4]).max() <= 1e-13 * max(np.abs(o[4]).max(), 1e-30)
+    assert np.abs(g[5] - o[5]).max() <= REL_TOL * max(np.abs(o[5]).max(), 1e-30)
