@@ -5,7 +5,8 @@
 // with IEEE division bit for bit over random finite inputs of every
 // exponent in the normal range, over inputs built next to multiples of the
 // divisor (quotients with a zero, one-third and two-thirds fractional ulp),
-// over signed zeros and infinities, and over a NaN.
+// over signed zeros and infinities, and over a NaN.  Quotients, which replaces
+// divisions by one value, is compared over random divisors too.
 #include "adc_internal.cuh"
 
 namespace adc {
@@ -39,6 +40,22 @@ __global__ void k_selftest_div(long long n, unsigned long long seed, unsigned lo
     if (k == 2) x = __longlong_as_double(0x7FF0000000000000ll);    // +inf
     if (k == 3) x = __longlong_as_double((long long)0xFFF0000000000000ull);  // -inf
     if (k == 4) x = __longlong_as_double(0x7FF8000000000000ll);    // NaN
+    {   // a random divisor: what Quotients accepts has the bits of the division
+      const unsigned long long g = splitmix(h);
+      const unsigned long long ey = 1023 - 340 + (g >> 52) % 681;
+      double y = __longlong_as_double((long long)((g & 0x800FFFFFFFFFFFFFull) | (ey << 52)));
+      if (k % 5 == 0) y = __longlong_as_double(__double_as_longlong(y) | 0x000FFFFFFFFFFF00ll);   // long runs of ones
+      bool bad = false;
+      const Quotients by(y, bad);
+      // the exponents that are taken, one in two times
+      double z = (g & 1) ? x : ldexp(x, -(int)((h >> 52) % 2001) + 1000 + (int)(g % 500) - 250);
+      if (k % 7 == 0) z = y * (double)(int)(g >> 40);   // exact and nearly exact quotients
+      const double f = by(z, bad);
+      if (!bad && __double_as_longlong(f) != __double_as_longlong(z / y)) ++local;
+      // and nothing within its range is refused
+      if (bad && (z == 0.0 || (fabs(z) >= 0x1p-299 && fabs(z) <= 0x1p299)) && fabs(y) >= 0x1p-299 && fabs(y) <= 0x1p299)
+        ++local;
+    }
     const double q3 = x / 3.0, q6 = x / 6.0, q12 = x / 12.0;
     if (isnan(x)) {   // a NaN must stay a NaN (payload bits are not compared)
       local += !isnan(div3(x)) + !isnan(div6(x)) + !isnan(div12(x));

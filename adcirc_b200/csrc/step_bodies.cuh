@@ -358,8 +358,9 @@ __device__ __forceinline__ void item_bc(const adc_ctx &c, double EP, int t) {
 // ----------------------------------------------------------------- RHS
 // gwce.F:1000-1617 for the 32 elements from e0, one per lane, IM=0 branches.
 // `sh`: 96 values of the warp.
-template <class R>
-__device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
+template <class R, bool kFast>
+__device__ __forceinline__ bool warp_rhs_by(const adc_ctx &c, int e0, R *sh) {
+  bool bad = false;
   const int nvalid = min(32, c.ne - e0);
   // idle lanes recompute the last element; not stored
   const int e = min(e0 + (int)(threadIdx.x & 31), c.ne - 1);
@@ -369,7 +370,8 @@ __device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
   // gives the same bits
   const bool dt2 = c.dt_pow2 != 0;
   const R IDT = R(c.inv_dt);
-  auto odt = [&](R x) { return dt2 ? x * IDT : x / DT; };
+  const Divisor<R, kFast> by_dt(DT, IDT, bad);
+  auto odt = [&](R x) { return dt2 ? x * IDT : by_dt(x, bad); };
   int n1 = c.nm[3 * e], n2 = c.nm[3 * e + 1], n3 = c.nm[3 * e + 2];
   int NCEle = c.nodecode[n1] * c.nodecode[n2] * c.nodecode[n3] * c.noff[e];
   R E0N1 = c.eta1[n1], E0N2 = c.eta1[n2], E0N3 = c.eta1[n3];
@@ -405,6 +407,11 @@ __device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
   R AreaIE2 = c.areas[e];
   R AreaIE = AreaIE2 / R(2.0);
   R AreaIE4 = R(2.0) * AreaIE2;
+  const Divisor<R, kFast> by_area(AreaIE2, bad);
+  auto by_area2x = [&](R x) {   // a power of two more: the half of the quotient
+    if constexpr (kFast && sizeof(R) == 8) return R(0.5) * by_area(x, bad);
+    return x / AreaIE4;
+  };
   R FDX1 = c.fdx[3 * e], FDX2 = c.fdx[3 * e + 1], FDX3 = c.fdx[3 * e + 2];
   R FDY1 = c.fdy[3 * e], FDY2 = c.fdy[3 * e + 1], FDY3 = c.fdy[3 * e + 2];
   R E0XGrad2A, E0YGrad2A, E1XGrad2A, E1YGrad2A, E1SQXGrad2A, E1SQYGrad2A;
@@ -430,15 +437,15 @@ __device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
   }
   R Tau0XGrad2A = T0N1 * FDX1 + T0N2 * FDX2 + T0N3 * FDX3;
   R Tau0YGrad2A = T0N1 * FDY1 + T0N2 * FDY2 + T0N3 * FDY3;
-  R EVMXGrad = (EVMN1 * FDX1 + EVMN2 * FDX2 + EVMN3 * FDX3) / AreaIE2;
-  R EVMYGrad = (EVMN1 * FDY1 + EVMN2 * FDY2 + EVMN3 * FDY3) / AreaIE2;
+  R EVMXGrad = by_area(EVMN1 * FDX1 + EVMN2 * FDX2 + EVMN3 * FDX3, bad);
+  R EVMYGrad = by_area(EVMN1 * FDY1 + EVMN2 * FDY2 + EVMN3 * FDY3, bad);
   R EVMAvgODT = odt(div3(EVMN1 + EVMN2 + EVMN3));
-  R MX = (EVMXGrad * (QX1N1 * FDX1 + QX1N2 * FDX2 + QX1N3 * FDX3) +
+  R MX = by_area(EVMXGrad * (QX1N1 * FDX1 + QX1N2 * FDX2 + QX1N3 * FDX3) +
                EVMYGrad * (QY1N1 * FDX1 + QY1N2 * FDX2 + QY1N3 * FDX3) -
-               EVMAvgODT * (ESN1 * FDX1 + ESN2 * FDX2 + ESN3 * FDX3)) / AreaIE2;
-  R MY = (EVMXGrad * (QX1N1 * FDY1 + QX1N2 * FDY2 + QX1N3 * FDY3) +
+               EVMAvgODT * (ESN1 * FDX1 + ESN2 * FDX2 + ESN3 * FDX3), bad);
+  R MY = by_area(EVMXGrad * (QX1N1 * FDY1 + QX1N2 * FDY2 + QX1N3 * FDY3) +
                EVMYGrad * (QY1N1 * FDY1 + QY1N2 * FDY2 + QY1N3 * FDY3) -
-               EVMAvgODT * (ESN1 * FDY1 + ESN2 * FDY2 + ESN3 * FDY3)) / AreaIE2;
+               EVMAvgODT * (ESN1 * FDY1 + ESN2 * FDY2 + ESN3 * FDY3), bad);
   R CorifAvg = div3(c.corif[n1] + c.corif[n2] + c.corif[n3]);
   R Tau0Avg = div3(T0N1 + T0N2 + T0N3);
   R Tau0QXAvg = div3(T0N1 * QX1N1 + T0N2 * QX1N2 + T0N3 * QX1N3);
@@ -450,11 +457,11 @@ __device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
   R ESAvg = div3(ESN1 + ESN2 + ESN3);
   R DPAvg = div3(c.dp[n1] + c.dp[n2] + c.dp[n3]);
   R al = c.alphal[e];
-  R GDPAvgOAreaIE4 = al * G * DPAvg / AreaIE4;
+  R GDPAvgOAreaIE4 = by_area2x(al * G * DPAvg);
   R GDPAvgOAreaIE4_S0 = GDPAvgOAreaIE4;   // DPAvgS0 == DPAvg when IFNL_HDP = 0
   R HAvg = div3(H1N1 + H1N2 + H1N3);
   R GHAvg = al * G * HAvg;
-  R GHAvgOAreaIE2 = GHAvg / AreaIE2;
+  R GHAvgOAreaIE2 = by_area(GHAvg, bad);
   R BSXAvg = div3(BSXN1 + BSXN2 + BSXN3);
   R BSYAvg = div3(BSYN1 + BSYN2 + BSYN3);
   R WSXAvg = R(0.0), WSYAvg = R(0.0);
@@ -463,7 +470,7 @@ __device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
     WSYAvg = div3(c.wsy1[n1] + c.wsy1[n2] + c.wsy1[n3]);
   }
   R MsFacR = div12(odt(AreaIE * ((dt2 ? IDT : R(1.0) / DT) - Tau0Avg / R(2.0))));
-  R GOAreaIE4 = al * G / AreaIE4;
+  R GOAreaIE4 = by_area2x(al * G);
   R Tau0SpaVar = div6(QX1Avg * Tau0XGrad2A + QY1Avg * Tau0YGrad2A);
   R A00pB00 = A00 + B00;
   R fa = p.ifnlfa * GOAreaIE4;
@@ -473,11 +480,11 @@ __device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
   R JYAvg = -CorifAvg * QX1Avg - fa * E1SQYGrad2A -
                  GHAvgOAreaIE2 * (Pr1N1 * FDY1 + Pr1N2 * FDY2 + Pr1N3 * FDY3) + WSYAvg -
                  BSYAvg + MY + Tau0QYAvg;
-  JXAvg = JXAvg - p.ifnlct * (QX1Avg * (U1N1 * FDX1 + U1N2 * FDX2 + U1N3 * FDX3) +
-                              QY1Avg * (U1N1 * FDY1 + U1N2 * FDY2 + U1N3 * FDY3)) / AreaIE2 +
+  JXAvg = JXAvg - by_area(p.ifnlct * (QX1Avg * (U1N1 * FDX1 + U1N2 * FDX2 + U1N3 * FDX3) +
+                              QY1Avg * (U1N1 * FDY1 + U1N2 * FDY2 + U1N3 * FDY3)), bad) +
           odt(p.ifnlcat * U1Avg * ESAvg);
-  JYAvg = JYAvg - p.ifnlct * (QX1Avg * (V1N1 * FDX1 + V1N2 * FDX2 + V1N3 * FDX3) +
-                              QY1Avg * (V1N1 * FDY1 + V1N2 * FDY2 + V1N3 * FDY3)) / AreaIE2 +
+  JYAvg = JYAvg - by_area(p.ifnlct * (QX1Avg * (V1N1 * FDX1 + V1N2 * FDX2 + V1N3 * FDX3) +
+                              QY1Avg * (V1N1 * FDY1 + V1N2 * FDY2 + V1N3 * FDY3)), bad) +
           odt(p.ifnlcat * V1Avg * ESAvg);
   R c0 = GDPAvgOAreaIE4_S0, c1 = GDPAvgOAreaIE4;
   R T1 = (2 * ESN1 + 1 * (ESN2 + ESN3)) * MsFacR -
@@ -495,6 +502,15 @@ __device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
   R nc = (R)NCEle;
   const R o[3] = {T1 * nc, T2 * nc, T3 * nc};
   warp_store_k<3>(reinterpret_cast<R *>(c.ebuf) + 3 * (size_t)e0, o, nvalid, sh);
+  return bad;
+}
+
+template <class R>
+__device__ __forceinline__ void warp_rhs(const adc_ctx &c, int e0, R *sh) {
+  if constexpr (sizeof(R) == 8) {
+    if (!__any_sync(0xffffffffu, warp_rhs_by<R, true>(c, e0, sh))) return;
+  }
+  warp_rhs_by<R, false>(c, e0, sh);
 }
 
 // GWCE_LV gather (element order) fused with gwce.F:1622-1631.
@@ -973,8 +989,9 @@ __device__ __forceinline__ double elem_alpha(const adc_ctx &c, int e) {
 // Element terms (momentum.F:298-699) for the 32 elements from e0, one per
 // lane.  `sh`: 192 values of the warp.  `alpha`: ALPHAL is formed here
 // (computeAlpha ends the wet/dry step that precedes).
-template <class R>
-__device__ __forceinline__ void warp_mom(const adc_ctx &c, int e0, R *sh, bool alpha) {
+template <class R, bool kFast>
+__device__ __forceinline__ bool warp_mom_by(const adc_ctx &c, int e0, R *sh, bool alpha) {
+  bool bad = false;
   const int nvalid = min(32, c.ne - e0);
   const int e = min(e0 + (int)(threadIdx.x & 31), c.ne - 1);   // idle lanes are not stored
   const adc_params_t &p = c.p;
@@ -1049,21 +1066,32 @@ __device__ __forceinline__ void warp_mom(const adc_ctx &c, int e0, R *sh, bool a
   R DBTPDYA = R(0.5) * (DBTPDY1A + DBTPDY2A);
   R ADVX = U1Avg * DU1DXA + V1Avg * DU1DYA;
   R ADVY = U1Avg * DV1DXA + V1Avg * DV1DYA;
-  R DU1DX = DU1DXA / AreaIE, DU1DY = DU1DYA / AreaIE;
-  R DV1DX = DV1DXA / AreaIE, DV1DY = DV1DYA / AreaIE;
+  const Divisor<R, kFast> by_area(AreaIE, bad);
+  R DU1DX = by_area(DU1DXA, bad), DU1DY = by_area(DU1DYA, bad);
+  R DV1DX = by_area(DV1DXA, bad), DV1DY = by_area(DV1DYA, bad);
+  const Divisor<R, kFast> by_h1(H1N1, bad), by_h2(H1N2, bad), by_h3(H1N3, bad);
   R EH1 = EVMEle * H1N1, EH2 = EVMEle * H1N2, EH3 = EVMEle * H1N3;
   R nc = (R)NCEle;
   R fct = nc * DT;
   R ax = -p.ifnlct * ADVX - GO2 * DBTPDXA - R(0.0);
   R ay = -p.ifnlct * ADVY - GO2 * DBTPDYA - R(0.0);
   R o[6];
-  o[0] = fct * (ax - (R(1.5) * ((EH1 * DU1DX) * FDX1 + (EH1 * DU1DY) * FDY1)) / H1N1);
-  o[1] = fct * (ax - (R(1.5) * ((EH2 * DU1DX) * FDX2 + (EH2 * DU1DY) * FDY2)) / H1N2);
-  o[2] = fct * (ax - (R(1.5) * ((EH3 * DU1DX) * FDX3 + (EH3 * DU1DY) * FDY3)) / H1N3);
-  o[3] = fct * (ay - (R(1.5) * ((EH1 * DV1DX) * FDX1 + (EH1 * DV1DY) * FDY1)) / H1N1);
-  o[4] = fct * (ay - (R(1.5) * ((EH2 * DV1DX) * FDX2 + (EH2 * DV1DY) * FDY2)) / H1N2);
-  o[5] = fct * (ay - (R(1.5) * ((EH3 * DV1DX) * FDX3 + (EH3 * DV1DY) * FDY3)) / H1N3);
+  o[0] = fct * (ax - by_h1(R(1.5) * ((EH1 * DU1DX) * FDX1 + (EH1 * DU1DY) * FDY1), bad));
+  o[1] = fct * (ax - by_h2(R(1.5) * ((EH2 * DU1DX) * FDX2 + (EH2 * DU1DY) * FDY2), bad));
+  o[2] = fct * (ax - by_h3(R(1.5) * ((EH3 * DU1DX) * FDX3 + (EH3 * DU1DY) * FDY3), bad));
+  o[3] = fct * (ay - by_h1(R(1.5) * ((EH1 * DV1DX) * FDX1 + (EH1 * DV1DY) * FDY1), bad));
+  o[4] = fct * (ay - by_h2(R(1.5) * ((EH2 * DV1DX) * FDX2 + (EH2 * DV1DY) * FDY2), bad));
+  o[5] = fct * (ay - by_h3(R(1.5) * ((EH3 * DV1DX) * FDX3 + (EH3 * DV1DY) * FDY3), bad));
   warp_store_k<6>(reinterpret_cast<R *>(c.ebuf) + 6 * (size_t)e0, o, nvalid, sh);
+  return bad;
+}
+
+template <class R>
+__device__ __forceinline__ void warp_mom(const adc_ctx &c, int e0, R *sh, bool alpha) {
+  if constexpr (sizeof(R) == 8) {
+    if (!__any_sync(0xffffffffu, warp_mom_by<R, true>(c, e0, sh, alpha))) return;
+  }
+  warp_mom_by<R, false>(c, e0, sh, alpha);
 }
 
 // gfortran's inline NORM2 for TKM(:,i) (scaled sum of squares starting
@@ -1088,8 +1116,9 @@ __device__ inline double norm2_3(const double *x) {
 
 
 // Nodal load, boundary condition and solve (momentum.F:713-1182).
-template <class R>
-__device__ __forceinline__ void node_mom(const adc_ctx &c, int i) {
+template <class R, bool kFast>
+__device__ __forceinline__ bool node_mom_by(const adc_ctx &c, int i) {
+  bool bad = false;
   const adc_params_t &p = c.p;
   const double DTO2 = p.dt / 2.0;
   const R *eb = reinterpret_cast<const R *>(c.ebuf);
@@ -1118,14 +1147,16 @@ __device__ __forceinline__ void node_mom(const adc_ctx &c, int i) {
   int NCI = c.nodecode[i];
   double ta = c.totalarea[i];
   if (ta != 0.0) {
-    mx = mx / ta;
-    my = my / ta;
+    const Divisor<double, kFast> by(ta, bad);
+    mx = by(mx, bad);
+    my = by(my, bad);
   }
   double uu1 = c.uu1[i], vv1 = c.vv1[i];
   double WSX = 0.0, WSY = 0.0;
   if (p.nws != 0) {
-    WSX = DTO2 * p.ifwind * (c.wsx1[i] / c.h1[i] + c.wsx2[i] / c.h2[i]);
-    WSY = DTO2 * p.ifwind * (c.wsy1[i] / c.h1[i] + c.wsy2[i] / c.h2[i]);
+    const Divisor<double, kFast> by_h1(c.h1[i], bad), by_h2(c.h2[i], bad);
+    WSX = DTO2 * p.ifwind * (by_h1(c.wsx1[i], bad) + by_h2(c.wsx2[i], bad));
+    WSY = DTO2 * p.ifwind * (by_h1(c.wsy1[i], bad) + by_h2(c.wsy2[i], bad));
   }
   const double *tkm = c.tkm + 3 * i;
   double VXX = DTO2 * (tkm[0] + 0.0);
@@ -1201,13 +1232,20 @@ __device__ __forceinline__ void node_mom(const adc_ctx &c, int i) {
   c.mom_x[i] = mx;
   c.mom_y[i] = my;
   double DDU = a1 * a2 - a3 * a4;
-  double u2 = (mx * a2 - my * a3) / DDU;
-  double v2 = (my * a1 - mx * a4) / DDU;
+  const Divisor<double, kFast> by_det(DDU, bad);
+  double u2 = by_det(mx * a2 - my * a3, bad);
+  double v2 = by_det(my * a1 - mx * a4, bad);
   c.uu2[i] = u2;
   c.vv2[i] = v2;
   double h2 = c.h2[i];
   c.qx2[i] = u2 * h2;
   c.qy2[i] = v2 * h2;
+  return bad;
+}
+
+template <class R>
+__device__ __forceinline__ void node_mom(const adc_ctx &c, int i) {
+  if (node_mom_by<R, true>(c, i)) node_mom_by<R, false>(c, i);
 }
 
 // Zero normal velocity gradient (IBTYPE 40), momentum.F:1157-1174: after
