@@ -16,9 +16,11 @@
 // took eleven launches of 1.5 to 2 us each on meshes too small to fill the
 // GPU, and two more passes over the elements' NM, NOFF and ALPHAL.  Measured
 // with the folds into the solve and the momentum passes (23 launches a step to
-// 13): 96 -> 88 us a step on the 2,500-node beach, 136 -> 125 us on a
-// 25k-node shelf, 0.68 -> 0.67 ms on one of 600k.
+// 13): 83 -> 76 us a step on the 533-node beach, 156 -> 143 us on a 25k-node
+// shelf.
 #include "step_bodies.cuh"
+
+#include <algorithm>
 
 namespace adc {
 
@@ -34,12 +36,13 @@ __global__ void __launch_bounds__(kThreads) k_step_begin(adc_ctx c, const adc_st
       v = *c.vstate;
       past = vortex_advance(c, st.timeloc, v);
     }
-    __syncthreads();
   }
+  // the other warps' shift hides the first thread's chain of divisions
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < c.np) {
-    node_shift(c, st, i, whole != 0, c.vortex_on != 0);
-    if (c.vortex_on) node_vortex(c, v, st.rampmete, i);
+  if (i < c.np) node_shift(c, st, i, whole != 0, c.vortex_on != 0);
+  if (c.vortex_on) {
+    __syncthreads();
+    if (i < c.np) node_vortex(c, v, st.rampmete, i);
   }
   // every block has read the old state before it takes its ticket
   if (c.vortex_on && threadIdx.x == 0 && atomicAdd(&c.tickets[0], 1) == (int)gridDim.x - 1) {
@@ -80,21 +83,55 @@ __global__ void k_lhs_drift_done(adc_ctx c) {
   w[1] = 0;
 }
 
-// Element pass.  The load-vector terms hold 128 registers; the matrix entries
-// of the few elements that change ride along.
-template <class R>
-__global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 3 : 2) k_gwce_elem(adc_ctx c) {
+// Element pass: matrix entries of the elements that change, or the pending
+// drift (kPart 1), the load-vector terms (kPart 2), or both (kPart 3).
+// Blocks of the load-vector terms: 64 threads, so that one block's gathers run
+// under another's arithmetic (600k nodes: 82 us, 88 with blocks of 256, 83
+// with 128), and a small mesh spreads over more SMs.  80 registers a thread
+// for half as many warps again was slower, 103 us.
+constexpr int kElemThreads = 64;
+constexpr int elem_threads(int part) { return part == 1 ? kThreads : kElemThreads; }
+
+template <class R, int kPart>
+__global__ void __launch_bounds__(elem_threads(kPart), kPart == 1 ? 4 : kThreads / kElemThreads * (sizeof(R) == 4 ? 3 : 2))
+    k_gwce_elem(adc_ctx c) {
   griddep_wait();
-  __shared__ R sh[kThreads / 32][32 * 3];
-  const bool rebuild = c.flags->ncchange > 0;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (rebuild) {
-    if (t < c.ne) elem_lhs<R>(c, t);
-  } else if (lhs_words(c)[1] && t < c.np) {
-    row_drift(c, t);
+  if (kPart & 1) {
+    if (c.flags->ncchange > 0) {
+      if (t < c.ne) elem_lhs<R>(c, t);
+    } else if (lhs_words(c)[1] && t < c.np) {
+      row_drift(c, t);
+    }
   }
-  const int e0 = t & ~31;
-  if (e0 < c.ne) warp_rhs<R>(c, e0, sh[threadIdx.x >> 5]);
+  if (kPart & 2) {
+    __shared__ R sh[kElemThreads / 32][32 * 3];
+    const int e0 = t & ~31;
+    if (e0 < c.ne) warp_rhs<R>(c, e0, sh[threadIdx.x >> 5]);
+  }
+}
+
+constexpr int kSMs = 148;
+
+// One kernel for both parts while its blocks run at once (512 threads of 128
+// registers on an SM).  Beyond that a second launch costs less than the first
+// part's memory passes at the second's occupancy: at 600k nodes 156 us
+// together, 21 + 82 us apart; on a small mesh a launch is some 2 us.
+template <class R>
+static void launch_elem(adc_ctx *c) {
+  const int nboth = std::max(c->ne, c->np);
+  const int nb = nblk(nboth, kElemThreads);
+  if (nb <= 2 * (kThreads / kElemThreads) * kSMs) {
+    launch_k(k_gwce_elem<R, 3>, nb, kElemThreads, c->stream, *c);
+  } else {
+    launch_k(k_gwce_elem<R, 1>, nblk(nboth), kThreads, c->stream, *c);
+    launch_k(k_gwce_elem<R, 2>, nblk(c->ne, kElemThreads), kElemThreads, c->stream, *c);
+    c->launches++;
+  }
+}
+void launch_gwce_elem(adc_ctx *c) {
+  if (f32_assembly(c)) launch_elem<float>(c);   // FP32 element assembly
+  else launch_elem<double>(c);
 }
 
 // EP = RMS of the diagonal (gwce.F:646-650) from the node blocks' partial
@@ -117,7 +154,7 @@ __device__ double ep_from_parts(const double *parts, int nparts, int np) {
 
 // Node pass.  The last block forms EP and settles the LHS words.
 template <class R>
-__global__ void __launch_bounds__(kThreads) k_gwce_node(adc_ctx c) {
+__global__ void __launch_bounds__(kThreads, 4) k_gwce_node(adc_ctx c) {
   griddep_wait();
   const int *words = lhs_words(c);
   const bool rebuild = c.flags->ncchange > 0;
@@ -174,8 +211,6 @@ __global__ void k_obc_rhs(adc_ctx c) {
   if (r < c.n_obc_rhs_nodes) bnd_obc(c, r);
 }
 
-template __global__ void k_gwce_elem<double>(adc_ctx);
-template __global__ void k_gwce_elem<float>(adc_ctx);
 template __global__ void k_gwce_node<double>(adc_ctx);
 template __global__ void k_gwce_node<float>(adc_ctx);
 

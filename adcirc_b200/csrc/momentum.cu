@@ -13,20 +13,24 @@
 
 namespace adc {
 
-// Four 256-thread blocks per SM (64 registers): measured 0.057 ms per
-// launch on the surge mesh against 0.062 ms at the compiler's choice (68).
+// 1,024 threads an SM (64 registers; with 768 threads of 80 the surge mesh's
+// launch takes 52 us instead of 46) in blocks of two warps, whose gathers and
+// arithmetic overlap better than those of eight (47 us).
+constexpr int kMomThreads = 64;
+
 template <class R>
-__global__ void __launch_bounds__(kThreads, 4) k_mom_elem(adc_ctx c, int alpha) {
+__global__ void __launch_bounds__(kMomThreads, 1024 / kMomThreads) k_mom_elem(adc_ctx c, int alpha) {
   griddep_wait();
-  __shared__ R sh[kThreads / 32][32 * 6];
+  __shared__ R sh[kMomThreads / 32][32 * 6];
   const int e0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31);
   if (e0 < c.ne) warp_mom<R>(c, e0, sh[threadIdx.x >> 5], alpha != 0);
 }
 
+// 64 registers: 39 us on the surge mesh, 44 with the compiler's 74.
 // With `log`, also the end of a step of adc_run: its iteration count and the
 // step table's cursor, which this kernel does not read.
 template <class R>
-__global__ void __launch_bounds__(kThreads) k_mom_node(adc_ctx c, int *log, int cap) {
+__global__ void __launch_bounds__(kThreads, 4) k_mom_node(adc_ctx c, int *log, int cap) {
   griddep_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < c.np) node_mom<R>(c, i);
@@ -44,12 +48,12 @@ int launch_momentum(adc_ctx *c, bool whole, int *log) {
   const int alpha = whole && c->p.nolifa == 2;
   kmark(c, KS_MOM_ELEM, 0);
   if (f32_momentum(c)) {   // FP32 element terms and their gather
-    launch_k(k_mom_elem<float>, nblk(c->ne), kThreads, c->stream, *c, alpha);
+    launch_k(k_mom_elem<float>, nblk(c->ne, kMomThreads), kMomThreads, c->stream, *c, alpha);
     kmark(c, KS_MOM_ELEM, 1);
     kmark(c, KS_MOM_NODE, 0);
     launch_k(k_mom_node<float>, nblk(c->np), kThreads, c->stream, *c, log, c->numitr_cap);
   } else {
-    launch_k(k_mom_elem<double>, nblk(c->ne), kThreads, c->stream, *c, alpha);
+    launch_k(k_mom_elem<double>, nblk(c->ne, kMomThreads), kMomThreads, c->stream, *c, alpha);
     kmark(c, KS_MOM_ELEM, 1);
     kmark(c, KS_MOM_NODE, 0);
     launch_k(k_mom_node<double>, nblk(c->np), kThreads, c->stream, *c, log, c->numitr_cap);

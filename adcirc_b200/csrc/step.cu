@@ -36,7 +36,7 @@ int jcg_setup_grid(adc_ctx *c, const JcgHostSell *h);
 // kernels defined in the other translation units
 __global__ void k_step_begin(adc_ctx c, const adc_step_t *steps, int whole);
 __global__ void k_apply_met(adc_ctx c);
-template <class R> __global__ void k_gwce_elem(adc_ctx c);
+void launch_gwce_elem(adc_ctx *c);
 template <class R> __global__ void k_gwce_node(adc_ctx c);
 __global__ void k_gwce_bc(adc_ctx c, const adc_step_t *steps);
 __global__ void k_obc_rhs(adc_ctx c);
@@ -66,24 +66,18 @@ int launch_shift_friction(adc_ctx *c, bool whole) {
 
 // Matrix and load vector, with their boundary rows.
 int launch_gwce(adc_ctx *c) {
-  const int nbe = nblk(std::max(c->ne, c->np)), nbn = nblk(c->np);
+  const int nbn = nblk(c->np);
   // the matrix entries and rows ride in the load vector's spans
   kmark(c, KS_LHS_ELEM, 0);
   kmark(c, KS_LHS_ELEM, 1);
   kmark(c, KS_LHS_GATHER, 0);
   kmark(c, KS_LHS_GATHER, 1);
   kmark(c, KS_RHS_ELEM, 0);
-  if (f32_assembly(c)) {   // FP32 element assembly
-    launch_k(k_gwce_elem<float>, nbe, kThreads, c->stream, *c);
-    kmark(c, KS_RHS_ELEM, 1);
-    kmark(c, KS_RHS_GATHER, 0);
-    launch_k(k_gwce_node<float>, nbn, kThreads, c->stream, *c);
-  } else {
-    launch_k(k_gwce_elem<double>, nbe, kThreads, c->stream, *c);
-    kmark(c, KS_RHS_ELEM, 1);
-    kmark(c, KS_RHS_GATHER, 0);
-    launch_k(k_gwce_node<double>, nbn, kThreads, c->stream, *c);
-  }
+  launch_gwce_elem(c);
+  kmark(c, KS_RHS_ELEM, 1);
+  kmark(c, KS_RHS_GATHER, 0);
+  if (f32_assembly(c)) launch_k(k_gwce_node<float>, nbn, kThreads, c->stream, *c);
+  else launch_k(k_gwce_node<double>, nbn, kThreads, c->stream, *c);
   kmark(c, KS_RHS_GATHER, 1);
   int rc = launch_flux_rhs(c);   // gwce.F:1737-1834, before the elevation rows
   if (rc) return rc;

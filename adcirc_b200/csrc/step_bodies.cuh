@@ -189,11 +189,22 @@ __device__ __forceinline__ void row_drift(const adc_ctx &c, int i) {
   const double winv_i = 1.0 / wi;
   const int s = i / kSlice, lane = i - s * kSlice;
   const int base = c.sl_ptr[s] + lane, len = c.rlen[i];
-  for (int k = 0; k < len; ++k) {
-    const int q = base + k * kSlice;
-    const double wj = c.jw[c.col[q]];
-    const double sv = c.offd[q] * wi * wj;
-    c.offd[q] = sv * winv_i * (1.0 / wj);
+  // a chunk's loads issue together: two round trips instead of two a slot
+  for (int kc = 0; kc < len; kc += kGatherChunk) {
+    double wj[kGatherChunk], v[kGatherChunk];
+#pragma unroll
+    for (int k = 0; k < kGatherChunk; ++k)
+      if (kc + k < len) {
+        const int q = base + (kc + k) * kSlice;
+        v[k] = c.offd[q];
+        wj[k] = c.jw[c.col[q]];
+      }
+#pragma unroll
+    for (int k = 0; k < kGatherChunk; ++k)
+      if (kc + k < len) {
+        const double sv = v[k] * wi * wj[k];
+        c.offd[base + (kc + k) * kSlice] = sv * winv_i * (1.0 / wj[k]);
+      }
   }
 }
 
