@@ -615,8 +615,8 @@ int jcg_setup_grid(adc_ctx *c, const JcgHostSell *h) {
 }
 
 // Empties the barrier lines: before every solve of jcg_kernel, and once for
-// newly allocated lines of the resident kernel, whose generations then go
-// on from solve to solve.
+// newly allocated lines of the resident and the ordered kernel, whose
+// generations then go on from solve to solve.
 void jcg_clear_barrier(adc_ctx *c) {
   const int nwords = (int)(2 * 128 * (size_t)c->jcg_rows_blocks / 8);
   launch_k(jcg_clear_lines, 8, 256, c->stream, (unsigned long long *)c->jlines, nwords);
@@ -665,15 +665,15 @@ int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int 
     c->launches++;
     return do_peror ? launch_jcg_peror(a, c) : ADC_OK;
   }
-  jcg_clear_barrier(c);
-  if (run_init) {
-    launch_k(jcg_init_kernel, 1, 1, c->stream, c->itp, c->bar, c->itmax);
-    c->launches++;
-  }
   if (c->jcg_res == 3) {
     if (int rc = launch_jcg_ordered(a, c)) return rc;
     c->launches++;
     return ADC_OK;
+  }
+  jcg_clear_barrier(c);
+  if (run_init) {
+    launch_k(jcg_init_kernel, 1, 1, c->stream, c->itp, c->bar, c->itmax);
+    c->launches++;
   }
   void *args[] = {&a};
   ADC_CUDA(cudaLaunchCooperativeKernel((const void *)jcg_kernel, dim3(c->jcg_grid), dim3(kThreads), args,
@@ -682,8 +682,8 @@ int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int 
   return ADC_OK;
 }
 
-// The time-step solve defers the COEF drift to the next GWCE.  `d1` (the
-// resident kernel only): D1 of the wet/dry pass after the elevation update.
+// The time-step solve defers the COEF drift to the next GWCE.  `d1` (not
+// jcg_kernel): D1 of the wet/dry pass after the elevation update.
 int launch_jcg(adc_ctx *c, int eta_update, bool d1) {
   // a mode with FP32 parts keeps no bitwise COEF history, so the drift is dropped
   return launch_jcg_impl(c, eta_update, 0, 1, any_f32(c) ? 2 : 1, d1);

@@ -143,16 +143,24 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
   const int nhalo = !scalar_block ? a.halo_ptr[blockIdx.x + 1] - a.halo_ptr[blockIdx.x] : 0;
   SlicePipe pipe{S_stage + (size_t)(2 * warp) * a.stage_bytes, &S_bar[2 * warp], S_meta, a.lcol,
                  a.flags, a.stage_bytes, s0, s1, s0 + warp, nwarps, lane, 0u, a.stage_wcap};
-  Rec *rec = &a.itp->rec;
   __shared__ ItpLocal L;              // used by the scalar block's thread 0 only
   __shared__ Rec s_rec;               // the record of the last reducing barrier
-  unsigned gen = 0;                   // barrier generation within this launch
-  if (threadIdx.x == 0) {   // every block steps its own copy of the ITPACK scalars
+  unsigned gen = a.bar->gen;          // barrier generation, going on from solve to solve
+  const int q1 = a.itp->q1;
+  if (threadIdx.x == 0) {
+    // Every block steps its own copy of the ITPACK scalars, from echall's
+    // start of a solve (itpackv.F:1212-1255, the zeta floor of jcg :223-232):
+    // cme is the last solve's until chgcon(0), q1 and rparm1 stay.
     const volatile Itp *g = a.itp;
-    L.zeta = g->zeta; L.cme = g->cme; L.gamma = g->gamma; L.rho = g->rho;
-    L.gamold = g->gamold; L.rhoold = g->rhoold; L.delnnm = g->delnnm; L.delsnm = g->delsnm;
-    L.udnm = g->udnm; L.stptst = g->stptst; L.cmold = g->cmold; L.rparm1 = g->rparm1;
-    L.itmax = g->itmax; L.adapt = g->adapt; L.q1 = g->q1; L.isym = g->isym; L.chg_ier = 0;
+    L.rparm1 = g->rparm1;
+    L.zeta = L.rparm1;
+    if (L.zeta < 512.0 * DBL_EPSILON) L.zeta = 512.0 * DBL_EPSILON;
+    L.cme = g->cme;
+    L.cmold = g->cmold;
+    L.gamold = g->gamold;
+    L.rhoold = g->rhoold;
+    L.delnnm = L.delsnm = L.gamma = L.rho = L.stptst = L.udnm = 0.0;
+    L.itmax = a.itmax; L.adapt = 1; L.q1 = q1; L.isym = 0; L.chg_ier = 0;
   }
   __syncthreads();
 
@@ -174,9 +182,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
     __syncwarp();
   };
 
-  // P2 needs the unorm flag of iteration 0, set before the launch.
-  Rec r = read_rec(rec);
-  const int need_u0 = r.need_unorm;
+  const int need_u0 = !q1;   // the norm of u at iteration 0
   double pd = 0.0, pt = 0.0, pu = 0.0;
   // Resident prologue.  Shared memory first holds, per row of the block
   // and per halo node, w = 1/sqrt(diag) and u' (P1), then d0 (P2).
@@ -344,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
   double *U[2] = {a.u1, a.u};
   int cur = 0;   // resident variant: S_dd half holding d(in)
   for (int in = 0; in < a.itmax; ++in) {
-    r = s_rec;
+    const Rec r = s_rec;
     if (r.halt) break;
     const double c1 = r.c1, c2 = r.c2, c3 = r.c3, c4 = r.c4;
     const int need_u = r.need_unorm;
@@ -438,43 +444,12 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
     });
     if (!ok) return;
   }
-  r = s_rec;
+  const Rec r = s_rec;
   const int fin = r.in;
   const double *usol = U[fin % 2];
 
-  // Optional peror (itpackv.F:607-720): the norms behind digit1/digit2.
-  // pmult (itpackv.F:1970-2005) forms c = u - sum_j coef(:,j) u(jcoef).
-  if (a.do_peror) {
-    double pb = 0.0, pr = 0.0;
-    for (int s = s0 + warp; s < s1; s += nwarps) {
-      int i = s * kSlice + lane;
-      if (i < n) {
-        double wv = a.w[i];
-        double wk = a.rhs[i] / wv;
-        pb += wk * wk;
-        int len = a.rlen[i];
-        int base = a.sl_ptr[s] + lane;
-        double cc = usol[i];
-        for (int k = 0; k < len; ++k) {
-          int idx = base + k * kSlice;
-          cc = cc - (double)sv_store[idx] * usol[a.col[idx]];
-        }
-        double wk2 = (a.rhs[i] - cc) / wv;
-        pr += wk2 * wk2;
-      }
-    }
-    bool ok = phase_reduce(a, scalar_block, gen, pb, pr, 0.0, 0.0,
-                           [&](double sb, double sr, double, double) {
-      if (scalar_block) {
-        a.itp->dtnrm = sb;
-        a.itp->unorm = sr;
-      }
-    });
-    if (!ok) return;
-  }
-
-  // Epilogue: unscal (itpackv.F:2447-2477) and the GWCE eta update
-  // (gwce.F:2006-2008).
+  // Epilogue: unscal (itpackv.F:2447-2477), the GWCE eta update
+  // (gwce.F:2006-2008) and wet/dry pass D1.
   for (int s = s0 + warp; s < s1; s += nwarps) {
     int i = s * kSlice + lane;
     if (i < n) {
@@ -482,7 +457,16 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
       double uf = usol[i] * wv;
       a.u[i] = uf;
       a.rhs[i] = a.rhs[i] * (1.0 / wv);
-      if (a.eta_update) a.eta2[i] = a.nodecode[i] * (uf + 0.0) + a.eta1[i];
+      if (a.eta_update) {
+        const int nc = a.nodecode[i];
+        double e2 = nc * (uf + 0.0) + a.eta1[i];
+        if (a.d1 && d1_dries(nc, a.dp[i], a.h0, e2)) {
+          a.nnodecode[i] = 0;
+          a.nodecode[i] = 0;
+          atomicAdd(&a.flags->ncchange, 1);
+        }
+        a.eta2[i] = e2;
+      }
     }
   }
   if (scalar_block && threadIdx.x == 0) {
@@ -492,9 +476,12 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
     g->zeta = L.zeta; g->cme = L.cme; g->gamma = L.gamma; g->rho = L.rho;
     g->gamold = L.gamold; g->rhoold = L.rhoold; g->delnnm = L.delnnm; g->delsnm = L.delsnm;
     g->udnm = L.udnm; g->stptst = L.stptst; g->cmold = L.cmold; g->rparm1 = L.rparm1;
+    g->sme = -1.0; g->itmax = L.itmax; g->isym = 0;
     g->adapt = L.adapt; g->q1 = L.q1; g->chg_ier = L.chg_ier;
     g->in = fin;
     g->halt = h;
+    a.bar->gen = gen;
+    if (a.d1) a.flags->n_w1_events = 0;
     if (a.defer_drift == 1) *a.drift_pending = 1;
     a.flags->numitr = fin;
     a.flags->ier = (h == 2) ? 13 : 0;

@@ -102,9 +102,9 @@ static int enqueue_step(adc_ctx *c, bool timed, int *log) {
   if ((rc = launch_gwce(c))) return rc;
   if ((rc = launch_warm_start(c))) return rc;
   if (timed) cudaEventRecordWithFlags(c->ev[2], c->stream, cudaEventRecordExternal);
-  // D1 of the wet/dry pass ends the resident solve, unless the predictor's
-  // training reads the solution first
-  const bool d1 = c->p.nolifa == 2 && (c->jcg_res == 1 || c->jcg_res == 2) && !predictor_trains(c);
+  // D1 of the wet/dry pass ends the solve (jcg_kernel apart), unless the
+  // predictor's training reads the solution first
+  const bool d1 = c->p.nolifa == 2 && c->jcg_res != 0 && !predictor_trains(c);
   if ((rc = launch_jcg(c, 1, d1))) return rc;
   if ((rc = launch_predictor_train(c))) return rc;   // nothing unless training is on
   if (timed) cudaEventRecordWithFlags(c->ev[3], c->stream, cudaEventRecordExternal);
