@@ -24,17 +24,18 @@
 // expects have come.  Measured on B200: about 500 cycles, against 2,700 to
 // 3,000 for an all-to-all through L2.
 //
-// Exchange, grid form (kGrid = 1): each block posts its two block sums as
-// one 16-byte word in its arrival line, and every block polls all lines.
-// Polling uses 128-bit atomics: a plain load that reaches L2
-// while the line is being written came back after 4,000 to 7,000 cycles
-// (148 blocks, either die), an atomic poll after 3,000.  An empty word holds
-// kEmpty, a signalling-NaN pattern no arithmetic produces.  A line has four
-// slots used in turn; a block empties slot (g + 2) & 3 when it posts
-// generation g and checks that this has been performed before it posts
-// g + 1.  Readers of g - 2 are done by then (everyone posted g - 1), and
+// Exchange, grid form (kGrid = 1): each block posts its block sums in a slot
+// of its arrival line, and every block polls all lines.  A poll is one
+// 32-byte load of a slot, which holds the sums of d.d, d.Ad and u.u; the
+// timeout flag, one word for the whole grid, is looked at once in 64 polls.
+// (128-bit atomic polls, with a second one for u.u and the flag read beside
+// each, made a step 139 us on a 25k-node shelf and 632 on one of 600k; it
+// takes 127 and 624.)  An empty word holds kEmpty, a signalling-NaN pattern
+// no arithmetic produces.  A line has four slots used in turn; a block empties
+// slot (g + 2) & 3 when it posts generation g and checks that this has been
+// performed before it posts g + 1.  Readers of g - 2 are done by then (everyone posted g - 1), and
 // nobody polls g + 2 before having seen everyone's g + 1.  Each line exists
-// twice, for even and odd blocks, which halves the atomics per address.  The
+// twice, for even and odd blocks, which halves the polls per address.  The
 // halo word is (dtwd, generation): a reader that finds an older generation
 // reads again, so the exchange needs no memory fence.  Generations go on
 // from solve to solve.  Every wait is bounded; on expiry the kernel records
@@ -110,17 +111,14 @@ __device__ __forceinline__ W2 exch_w2(void *p, unsigned long long x, unsigned lo
   return r;
 }
 
-// Reads a 16-byte word as an atomic (compares with kEmpty words and writes
-// the same back).
-__device__ __forceinline__ W2 poll_w2(void *p) {
-  W2 r;
-  asm volatile(
-      "{\n .reg .b128 r, s;\n mov.b128 r, {%3, %3};\n"
-      " atom.relaxed.gpu.global.cas.b128 s, [%2], r, r;\n mov.b128 {%0, %1}, s;\n}\n"
-      : "=l"(r.x), "=l"(r.y)
-      : "l"(p), "l"(kEmpty)
-      : "memory");
-  return r;
+// One poll of a slot: its first three words, each single-copy atomic.
+__device__ __forceinline__ void poll_slot(const void *p, unsigned long long &x, unsigned long long &y,
+                                          unsigned long long &z) {
+  [[maybe_unused]] unsigned long long w;
+  asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(x), "=l"(y), "=l"(z), "=l"(w)
+               : "l"(p)
+               : "memory");
 }
 
 __device__ __forceinline__ uint32_t cluster_addr(const void *p, int rank) {
@@ -553,9 +551,11 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
   auto halo_wait = [&](const char *p, W2 q, unsigned g) -> double {
     if (q.y != g) {
       const long long tw = clock64();
+      unsigned polls = 0;
       do {
         q = ld_w2(p);
-        if (q.y != g && (clock64() - tw > kSpinCycles || *(volatile int *)&a.flags->timeout)) {
+        if (q.y != g && ++polls % 64 == 0 &&
+            (clock64() - tw > kSpinCycles || *(volatile int *)&a.flags->timeout)) {
           atomicExch(&a.flags->timeout, 1);
           bad = 1;
           break;
@@ -814,25 +814,16 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
             char *line = (char *)a.arrive + ((size_t)(b & 1) * nrb + q) * 128 + slot;
             const long long tw = clock64();
             W2 y, z = {0ull, 0ull};
-            for (;;) {
-              y = poll_w2(line);
-              if (y.x != kEmpty && y.y != kEmpty) break;
-              if (clock64() - tw > kSpinCycles || *(volatile int *)&a.flags->timeout) {
+            for (unsigned polls = 1;; ++polls) {
+              poll_slot(line, y.x, y.y, z.x);
+              if (y.x != kEmpty && y.y != kEmpty && (!need_u || z.x != kEmpty)) break;
+              if (polls % 64 == 0 && (clock64() - tw > kSpinCycles || *(volatile int *)&a.flags->timeout)) {
                 atomicExch(&a.flags->timeout, 1);
                 bad = 1;
                 break;
               }
             }
-            if (need_u)
-              for (;;) {
-                z = poll_w2(line + 16);
-                if (z.x != kEmpty) break;
-                if (clock64() - tw > kSpinCycles || *(volatile int *)&a.flags->timeout) {
-                  atomicExch(&a.flags->timeout, 1);
-                  bad = 1;
-                  break;
-                }
-              }
+            if (!need_u) z.x = 0ull;
             sd += bitsd(y.x);
             st += bitsd(y.y);
             su += bitsd(z.x);
