@@ -121,13 +121,19 @@ template <class R>
 static void launch_elem(adc_ctx *c) {
   const int nboth = std::max(c->ne, c->np);
   const int nb = nblk(nboth, kElemThreads);
+  kmark(c, KS_LHS_ELEM, 0);
   if (nb <= 2 * (kThreads / kElemThreads) * kSMs) {
+    kmark(c, KS_LHS_ELEM, 1);
+    kmark(c, KS_RHS_ELEM, 0);
     launch_k(k_gwce_elem<R, 3>, nb, kElemThreads, c->stream, *c);
   } else {
     launch_k(k_gwce_elem<R, 1>, nblk(nboth), kThreads, c->stream, *c);
+    kmark(c, KS_LHS_ELEM, 1);
+    kmark(c, KS_RHS_ELEM, 0);
     launch_k(k_gwce_elem<R, 2>, nblk(c->ne, kElemThreads), kElemThreads, c->stream, *c);
     c->launches++;
   }
+  kmark(c, KS_RHS_ELEM, 1);
 }
 void launch_gwce_elem(adc_ctx *c) {
   if (f32_assembly(c)) launch_elem<float>(c);   // FP32 element assembly

@@ -67,14 +67,10 @@ int launch_shift_friction(adc_ctx *c, bool whole) {
 // Matrix and load vector, with their boundary rows.
 int launch_gwce(adc_ctx *c) {
   const int nbn = nblk(c->np);
-  // the matrix entries and rows ride in the load vector's spans
-  kmark(c, KS_LHS_ELEM, 0);
-  kmark(c, KS_LHS_ELEM, 1);
+  launch_gwce_elem(c);
+  // the matrix rows are gathered in the load vector's span
   kmark(c, KS_LHS_GATHER, 0);
   kmark(c, KS_LHS_GATHER, 1);
-  kmark(c, KS_RHS_ELEM, 0);
-  launch_gwce_elem(c);
-  kmark(c, KS_RHS_ELEM, 1);
   kmark(c, KS_RHS_GATHER, 0);
   if (f32_assembly(c)) launch_k(k_gwce_node<float>, nbn, kThreads, c->stream, *c);
   else launch_k(k_gwce_node<double>, nbn, kThreads, c->stream, *c);

@@ -600,11 +600,14 @@ int adc_phase_times(adc_ctx *ctx, double *ms_shift, double *ms_gwce, double *ms_
 
 /* Device time (ms) of single kernels and passes of the last adc_timestep
  * (events inside its captured step graph), in this order; n entries are
- * written.  No reference counterpart (measurement only). */
-#define ADC_KT_LHS_ELEM 0     /* GWCE matrix element terms (gwce.F:427-592) */
-#define ADC_KT_LHS_GATHER 1   /* their node-centric gather into COEF */
+ * written.  No reference counterpart (measurement only).  The matrix rows are
+ * gathered with the load vector, and on meshes of up to one wave of elements
+ * their element terms are formed with its; a span whose work runs inside
+ * another is empty. */
+#define ADC_KT_LHS_ELEM 0     /* GWCE matrix element terms (gwce.F:427-592), or COEF's pending drift */
+#define ADC_KT_LHS_GATHER 1   /* empty: inside ADC_KT_RHS_GATHER */
 #define ADC_KT_RHS_ELEM 2     /* GWCE load-vector element terms (gwce.F:1000-1615) */
-#define ADC_KT_RHS_GATHER 3   /* their gather into GWCE_LV */
+#define ADC_KT_RHS_GATHER 3   /* their gather into GWCE_LV, and the matrix rows' into COEF */
 #define ADC_KT_JCG 4          /* the JCG solve (itpackv.F:63-604), all kernels */
 #define ADC_KT_WETDRY 5       /* computeWettingAndDrying + H2 (wetdry.F:140-1652) */
 #define ADC_KT_MOM_ELEM 6     /* momentum element terms (momentum.F:298-699) */
