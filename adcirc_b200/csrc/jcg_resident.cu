@@ -30,7 +30,7 @@
 // timeout flag, one word for the whole grid, is looked at once in 64 polls.
 // (128-bit atomic polls, with a second one for u.u and the flag read beside
 // each, made a step 139 us on a 25k-node shelf and 632 on one of 600k; it
-// takes 127 and 624.)  An empty word holds kEmpty, a signalling-NaN pattern
+// takes 130 and 624.)  An empty word holds kEmpty, a signalling-NaN pattern
 // no arithmetic produces.  A line has four slots used in turn; a block empties
 // slot (g + 2) & 3 when it posts generation g and checks that this has been
 // performed before it posts g + 1.  Readers of g - 2 are done by then (everyone posted g - 1), and
