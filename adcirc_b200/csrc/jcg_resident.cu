@@ -478,11 +478,12 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
 
   // The warp's streamed slices: bit k set where slice k is streamed.  The
   // q-th of them goes through buffer q & 1, and two copies are in flight,
-  // across the exchange too.
+  // across the exchange too.  With kRegs none is: what is not resident has no
+  // slots beyond the registers'.
   unsigned smask = 0u;
   uint32_t bar_par = 0u;
   int bad = 0;   // an expired wait of this thread
-  if (row_warp) {
+  if (row_warp && !kRegs) {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int ls = warp + k * kRowWarps;
@@ -1168,11 +1169,38 @@ static bool cluster16(const void *fn, size_t smem) {
   return ok;
 }
 
-// Chooses the launch shape for a matrix, builds its block-local tables and
-// uploads them; done = false where the resident kernel does not apply.
-int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
+// A launch shape and its block-local tables.
+struct ResShape {
+  int grid, nrb, k;   // form, row blocks, slices per warp of the instance
+  int rows_max, halo_max, stage;
+  int o[9];           // shared-memory offsets
+  size_t total;       // bytes of shared memory
+  std::vector<uint4> rcol;
+  std::vector<int4> meta;
+  std::vector<int> hptr, hids, pptr;
+  std::vector<int2> push;
+  std::vector<unsigned char> rle;
+};
+
+// Slices per warp of the instance for at most `k` (0: none).
+static int res_k(int k, bool grid) {
+  if (!grid) return k <= 1 ? 1 : k <= 2 ? 2 : 0;
+  return k <= 1 ? 1 : k <= 2 ? 2 : k <= 4 ? 4 : k <= 6 ? 6 : k <= 9 ? 9 : 0;
+}
+
+// Whether the instance reads a slice of width w from shared memory wherever
+// the planner has left it: kRegs' groups beyond the first.
+static bool reads_resident(int k, int w) { return k <= 2 && slot_groups(w) > 1; }
+
+// Fills `p` for a matrix of n rows, on the host alone: `limit(k, grid, bytes)`
+// gives the dynamic shared memory an instance may use, `cluster(k, bytes)`
+// whether 16 of its blocks can be a cluster.  done = false where the resident
+// kernel does not apply.
+template <class L, class F>
+static int resident_shape(int n, const JcgHostSell *h, int itmax, int nrb_req, int nsm, L limit, F cluster,
+                          ResShape &p, bool &done) {
   done = false;
-  const int n = c->np, nsl = c->nslices;
+  const int nsl = (n + kSlice - 1) / kSlice;
   int wmax = 1;
   for (int s = 0; s < nsl; ++s) wmax = std::max(wmax, h->sl_w[s]);
   if (wmax >= 128) return ADC_OK;
@@ -1180,8 +1208,8 @@ int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
   // four (24,963 rows) an iteration took 4.2 us in the cluster.  Beyond, one
   // block per SM, with at least one slice per warp.
   int grid = 1, nrb = std::max(1, std::min(nsm, (nsl + kRowWarps - 1) / kRowWarps));
-  if (c->jcg_nrb_req > 0) nrb = std::max(1, std::min({c->jcg_nrb_req, nsm, nsl}));
-  if (c->jcg_nrb_req == 0) {
+  if (nrb_req > 0) nrb = std::max(1, std::min({nrb_req, nsm, nsl}));
+  if (nrb_req == 0) {
     int nb = 1;
     while (nb < kMaxCluster && nb * kRowWarps < nsl) nb *= 2;
     if (nsl <= nb * kRowWarps * 2) {
@@ -1189,18 +1217,21 @@ int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
       nrb = nb;
     }
   }
-  for (;;) {   // at most twice: cluster form, then grid form
+  int k_min = 1;
+  for (;;) {   // at most three times: cluster form, grid form, grid form from k_min
     int per = 0;
     for (int b = 0; b < nrb; ++b)
       per = std::max(per, block_begin(nsl, nrb, b + 1) - block_begin(nsl, nrb, b));
-    const int k = (per + kRowWarps - 1) / kRowWarps, rows_max = per * kSlice;
-    const void *fn = res_fn(k, grid != 0);
-    bool fits = fn != nullptr;
-    std::vector<uint4> rcol;
-    std::vector<int4> meta(nsl);
-    std::vector<int> hptr, hids, pptr(nrb + 1, 0);
-    std::vector<int2> push;
-    std::vector<unsigned char> rle;
+    const int k = res_k(std::max(k_min, (per + kRowWarps - 1) / kRowWarps), grid != 0), rows_max = per * kSlice;
+    bool fits = k != 0;
+    p = ResShape();
+    std::vector<uint4> &rcol = p.rcol;
+    std::vector<int4> &meta = p.meta;
+    std::vector<int> &hptr = p.hptr, &hids = p.hids, &pptr = p.pptr;
+    std::vector<int2> &push = p.push;
+    std::vector<unsigned char> &rle = p.rle;
+    meta.resize(nsl);
+    pptr.assign(nrb + 1, 0);
     int halo_max = 0;
     if (fits) {
       // block-local columns: a row of the block is its offset from the first
@@ -1264,18 +1295,18 @@ int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
     if (fits) {
       const size_t vb = (size_t)rows_max + halo_max + 1;   // and the zero cell
       size_t o = align_up(8 * vb, 128);
-      c->jr_o[0] = (int)o; o += align_up((grid ? 8 : 24) * (size_t)halo_max, 128);
-      c->jr_o[1] = (int)o; o += align_up(4 * (size_t)halo_max, 128);
-      c->jr_o[2] = (int)o; o += align_up(32 * (size_t)(c->itmax + 2), 128);
-      c->jr_o[3] = (int)o; o += align_up(16 * (size_t)per, 128);
-      c->jr_o[4] = (int)o; o += align_up(8 * (grid ? 6 : 9) * (size_t)kPart, 128);
-      c->jr_o[5] = (int)o; o += align_up(16 * kRowWarps, 128);
+      p.o[0] = (int)o; o += align_up((grid ? 8 : 24) * (size_t)halo_max, 128);
+      p.o[1] = (int)o; o += align_up(4 * (size_t)halo_max, 128);
+      p.o[2] = (int)o; o += align_up(32 * (size_t)(itmax + 2), 128);
+      p.o[3] = (int)o; o += align_up(16 * (size_t)per, 128);
+      p.o[4] = (int)o; o += align_up(8 * (grid ? 6 : 9) * (size_t)kPart, 128);
+      p.o[5] = (int)o; o += align_up(16 * kRowWarps, 128);
       int push_max = 0;
       for (int b = 0; b < nrb; ++b) push_max = std::max(push_max, pptr[b + 1] - pptr[b]);
-      c->jr_o[8] = (int)o; o += align_up(8 * (size_t)push_max, 128);
-      c->jr_o[6] = (int)o;
-      size_t limit = 0;
-      if (int rc = jcg_smem_limit(fn, &limit)) return rc;
+      p.o[8] = (int)o; o += align_up(8 * (size_t)push_max, 128);
+      p.o[6] = (int)o;
+      size_t room_max = 0;
+      if (int rc = limit(k, grid != 0, &room_max)) return rc;
       // columns and values of a slice, in whole groups of eight slots
       auto slice_bytes = [&](int w) { return (size_t)slot_groups(w) * (512 + 2048); };
       auto bytes = [&](int s) { return slice_bytes(h->sl_w[s]); };
@@ -1288,7 +1319,7 @@ int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
         all = std::max(all, t);
       }
       size_t area = align_up(area0, 128), stage = 0, room = all;
-      if (o + area + all > limit) {
+      if (o + area + all > room_max) {
         if (!grid) {
           fits = false;
         } else {
@@ -1300,11 +1331,11 @@ int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
           while (wcap > 1 && over + hist[wcap] <= nsl / 200) over += hist[wcap--];
           stage = align_up(slice_bytes(wcap), 128);
           area = align_up(std::max(area0, 2 * kRowWarps * stage), 128);
-          fits = o + area <= limit;
-          room = fits ? limit - o - area : 0;
+          fits = o + area <= room_max;
+          room = fits ? room_max - o - area : 0;
         }
       }
-      c->jr_o[7] = (int)(o + area);
+      p.o[7] = (int)(o + area);
       if (fits) {
         // residency: the odd slices of every warp first, so that a streamed
         // slice's copy runs while the warp works on a resident one
@@ -1326,39 +1357,69 @@ int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
           used_max = std::max(used_max, used);
         }
         total = o + area + used_max;
-        c->jcg_stage_bytes = (int)stage;
+        p.stage = (int)stage;
       }
     }
     // One block per SM fits by its launch bounds and the limit above, and so
     // does a cluster of up to eight; 16 are a device's choice.
-    if (fits && !grid && nrb > 8) fits = cluster16(fn, total);
+    if (fits && !grid && nrb > 8) fits = cluster(k, total);
     if (!fits) {
       if (grid) return ADC_OK;
       grid = 1;
       nrb = std::max(1, std::min(nsm, (nsl + kRowWarps - 1) / kRowWarps));
       continue;
     }
-    JcgTables T;
-    const size_t o_rcol = T.add(rcol), o_meta = T.add(meta), o_hptr = T.add(hptr), o_hids = T.add(hids),
-                 o_rle = T.add(rle), o_pptr = T.add(pptr), o_push = T.add(push);
-    if (int rc = T.upload(c)) return rc;
-    c->jrcol = (uint4 *)(c->jtab + o_rcol);
-    c->jmeta = (int4 *)(c->jtab + o_meta);
-    c->jhalo_ptr = (int *)(c->jtab + o_hptr);
-    c->jhalo_ids = (int *)(c->jtab + o_hids);
-    c->jrle = c->jtab + o_rle;
-    c->jpush_ptr = (int *)(c->jtab + o_pptr);
-    c->jpush = (int2 *)(c->jtab + o_push);
-    c->jcg_rows_blocks = nrb;
-    c->jcg_grid = nrb;
-    c->jcg_res = grid ? 1 : 2;
-    c->jcg_res_k = k;
-    c->jcg_rows_max = rows_max;
-    c->jcg_halo_max = halo_max;
-    c->jcg_smem = total;
+    // where shared memory ran out for slices that the instance would read
+    // there, the smallest that streams them or reads them in place
+    const auto misread = [k](const int4 &m) { return m.w < 0 && reads_resident(k, m.y); };
+    if (std::any_of(meta.begin(), meta.end(), misread)) {
+      k_min = 3;
+      continue;
+    }
+    p.grid = grid;
+    p.nrb = nrb;
+    p.k = k;
+    p.rows_max = rows_max;
+    p.halo_max = halo_max;
+    p.total = total;
     done = true;
     return ADC_OK;
   }
+}
+
+// Chooses the launch shape for a matrix, builds its block-local tables and
+// uploads them; done = false where the resident kernel does not apply.
+int plan_jcg_resident(adc_ctx *c, const JcgHostSell *h, int nsm, bool &done) {
+  ResShape p;
+  if (int rc = resident_shape(
+          c->np, h, c->itmax, c->jcg_nrb_req, nsm,
+          [](int k, bool grid, size_t *bytes) { return jcg_smem_limit(res_fn(k, grid), bytes); },
+          [](int k, size_t bytes) { return cluster16(res_fn(k, false), bytes); }, p, done))
+    return rc;
+  if (!done) return ADC_OK;
+  done = false;
+  JcgTables T;
+  const size_t o_rcol = T.add(p.rcol), o_meta = T.add(p.meta), o_hptr = T.add(p.hptr), o_hids = T.add(p.hids),
+               o_rle = T.add(p.rle), o_pptr = T.add(p.pptr), o_push = T.add(p.push);
+  if (int rc = T.upload(c)) return rc;
+  c->jrcol = (uint4 *)(c->jtab + o_rcol);
+  c->jmeta = (int4 *)(c->jtab + o_meta);
+  c->jhalo_ptr = (int *)(c->jtab + o_hptr);
+  c->jhalo_ids = (int *)(c->jtab + o_hids);
+  c->jrle = c->jtab + o_rle;
+  c->jpush_ptr = (int *)(c->jtab + o_pptr);
+  c->jpush = (int2 *)(c->jtab + o_push);
+  for (int q = 0; q < 9; ++q) c->jr_o[q] = p.o[q];
+  c->jcg_rows_blocks = p.nrb;
+  c->jcg_grid = p.nrb;
+  c->jcg_res = p.grid ? 1 : 2;
+  c->jcg_res_k = p.k;
+  c->jcg_rows_max = p.rows_max;
+  c->jcg_halo_max = p.halo_max;
+  c->jcg_stage_bytes = p.stage;
+  c->jcg_smem = p.total;
+  done = true;
+  return ADC_OK;
 }
 
 int launch_jcg_resident(const JcgArgs &a0, const adc_ctx *c) {
@@ -1403,3 +1464,33 @@ int launch_jcg_resident(const JcgArgs &a0, const adc_ctx *c) {
 }
 
 }  // namespace adc
+
+using namespace adc;
+
+extern "C" int adc_selftest_jcg_shape(int n, const int *sl_ptr, const int *sl_w, const int *col, const int *rlen,
+                                      int itmax, int row_blocks, int sms, int smem, int *out) {
+  if (n < 1 || !sl_ptr || !sl_w || !col || !rlen || itmax < 0 || !out) {
+    set_error("adc_selftest_jcg_shape: bad arguments");
+    return ADC_ERR_ARG;
+  }
+  const JcgHostSell h{sl_ptr, sl_w, col, rlen};
+  ResShape p;
+  bool done = false;
+  if (int rc = resident_shape(
+          n, &h, itmax, row_blocks, sms,
+          [smem](int, bool, size_t *bytes) {
+            *bytes = (size_t)smem;
+            return ADC_OK;
+          },
+          [](int, size_t) { return true; }, p, done))
+    return rc;
+  out[0] = !done ? 0 : p.grid ? 1 : 2;
+  out[1] = done ? p.k : 0;
+  out[2] = out[3] = 0;
+  for (const int4 &m : p.meta)
+    if (done && m.w < 0) {
+      ++out[2];
+      if (reads_resident(p.k, m.y)) ++out[3];
+    }
+  return ADC_OK;
+}

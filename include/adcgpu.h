@@ -469,6 +469,15 @@ int adc_hotstart_read(adc_ctx *ctx, const char *path);
  * (used in the FP64 element kernels) differs in any bit from IEEE division. */
 int adc_selftest_div_const(long long n, unsigned long long seed, long long *mismatches);
 
+/* The resident JCG kernel's launch shape for a sliced-ELL matrix (32-row
+ * slices: first slot and width of each; per slot the 0-based column; row
+ * lengths), ITMAX, requested row blocks (0: its own choice), SMs and shared
+ * memory per block, on the host alone: out[0] form (0 does not apply, 1 grid,
+ * 2 cluster), out[1] slices per warp, out[2] slices that are not resident,
+ * out[3] those of them that the instance would read as if they were (0). */
+int adc_selftest_jcg_shape(int n, const int *sl_ptr, const int *sl_w, const int *col, const int *rlen,
+                           int itmax, int row_blocks, int sms, int smem, int *out);
+
 /* Specified normal flux (NFLUXF = 1, IBTYPE 2/12/22 with NFFR > 0): uploads
  * the flux constituents once; every later step forms QN2 on the device
  * (timestep.F:861-880) after shifting QN0 <- QN1 <- QN2 (timestep.F:606-613),
