@@ -1,9 +1,10 @@
 // jcg.cu -- ITPACK 2D JCG (itpackv.F:63-604) as one persistent cooperative
 // kernel with its vectors in global memory, and the solver's set-up and
-// launch.  The resident kernel (jcg_resident.cu) serves every matrix whose
-// row blocks fit on the SMs; this one serves the rest (more than about
-// 650,000 rows, 128 or more neighbours) and adc_jcg_noalloc, which builds no
-// host tables.
+// launch.  Two kernels with block-local tables come first: jcg_resident.cu,
+// where a matrix fits on the SMs (639,360 rows at most), then jcg_ordered.cu
+// (about a million).  This one serves what neither takes (more rows, 128 or
+// more neighbours, many wide rows together with a large ITMAX) and
+// adc_jcg_noalloc, which builds no host tables.
 //
 // Design
 //  * The scaled system (scal, itpackv.F:2281-2421) is built in-kernel from
@@ -577,9 +578,12 @@ int jcg_smem_limit(const void *fn, size_t *limit) {
 }
 
 // Launch shape of the solver.  With host copies of the sliced ELL the
-// resident kernel is planned first; without them, or where it does not
-// apply, as many 256-thread row blocks as can be co-resident (2 per SM),
-// plus the scalar block.
+// resident kernel is planned first (not in the modes with FP32 parts), then
+// the ordered one; without them, or where neither applies, jcg_kernel with as
+// many 256-thread row blocks as can be co-resident (2 per SM), plus the scalar
+// block.  A step of an FP64 shelf takes 637 us at 620k nodes (resident), 746
+// at 660k and 1,137 at 800k (ordered; 1,190 and 1,373 with jcg_kernel), 1,523
+// at 1,000k (ordered; 1,676), 1,786 at 1,061k (jcg_kernel).
 int jcg_setup_grid(adc_ctx *c, const JcgHostSell *h) {
   int dev = 0, nsm = 0;
   ADC_CUDA(cudaGetDevice(&dev));
@@ -591,7 +595,10 @@ int jcg_setup_grid(adc_ctx *c, const JcgHostSell *h) {
   c->jcg_res = 0;
   if (h) {
     bool done = false;
-    if (int rc = any_f32(c) ? plan_jcg_ordered(c, h, nsm, done) : plan_jcg_resident(c, h, nsm, done)) return rc;
+    if (!any_f32(c))
+      if (int rc = plan_jcg_resident(c, h, nsm, done)) return rc;
+    if (!done)
+      if (int rc = plan_jcg_ordered(c, h, nsm, done)) return rc;
     if (done) return ADC_OK;
   }
   // keep at least ~8 slices per block so the barrier cost stays amortised
@@ -668,7 +675,7 @@ int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int 
   if (c->jcg_res == 3) {
     if (int rc = launch_jcg_ordered(a, c)) return rc;
     c->launches++;
-    return ADC_OK;
+    return do_peror ? launch_jcg_peror(a, c) : ADC_OK;
   }
   jcg_clear_barrier(c);
   if (run_init) {

@@ -1,5 +1,6 @@
-// jcg_common.cuh -- launch arguments of the two JCG kernels (jcg.cu,
-// jcg_resident.cu) and the host entry points of the resident one.
+// jcg_common.cuh -- launch arguments of the three JCG kernels (jcg.cu,
+// jcg_resident.cu, jcg_ordered.cu) and the host entry points of the two with
+// block-local tables.
 #pragma once
 
 #include "adc_internal.cuh"

@@ -1,6 +1,7 @@
-// jcg_ordered.cu -- ITPACK 2D JCG for the modes with FP32 parts.
+// jcg_ordered.cu -- ITPACK 2D JCG for the modes with FP32 parts, and in FP64
+// for matrices beyond the resident kernel (jcg_resident.cu).
 //
-// In those modes a last-bit change of a dot product changes, now and then,
+// In the modes with FP32 parts a last-bit change of a dot product changes, now and then,
 // how a value rounds to FP32, and from there a run's results at the 1e-6
 // level.  This kernel therefore keeps the summation tree those modes have
 // always had (256-thread row blocks, their block sums in block order), where
@@ -149,18 +150,19 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
   const int q1 = a.itp->q1;
   if (threadIdx.x == 0) {
     // Every block steps its own copy of the ITPACK scalars, from echall's
-    // start of a solve (itpackv.F:1212-1255, the zeta floor of jcg :223-232):
-    // cme is the last solve's until chgcon(0), q1 and rparm1 stay.
+    // start of a solve (itpackv.F:1212-1255, the zeta floor of jcg :223-232)
+    // or, without run_init, from the caller's: cme is the last solve's until
+    // chgcon(0), q1 and rparm1 stay.
     const volatile Itp *g = a.itp;
     L.rparm1 = g->rparm1;
-    L.zeta = L.rparm1;
-    if (L.zeta < 512.0 * DBL_EPSILON) L.zeta = 512.0 * DBL_EPSILON;
+    L.zeta = a.run_init ? L.rparm1 : g->zeta;
+    if (a.run_init && L.zeta < 512.0 * DBL_EPSILON) L.zeta = 512.0 * DBL_EPSILON;
     L.cme = g->cme;
     L.cmold = g->cmold;
     L.gamold = g->gamold;
     L.rhoold = g->rhoold;
     L.delnnm = L.delsnm = L.gamma = L.rho = L.stptst = L.udnm = 0.0;
-    L.itmax = a.itmax; L.adapt = 1; L.q1 = q1; L.isym = 0; L.chg_ier = 0;
+    L.itmax = a.itmax; L.adapt = a.run_init ? 1 : g->adapt; L.q1 = q1; L.isym = 0; L.chg_ier = 0;
   }
   __syncthreads();
 
@@ -454,7 +456,12 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
     int i = s * kSlice + lane;
     if (i < n) {
       double wv = a.w[i];
-      double uf = usol[i] * wv;
+      const double us = usol[i];
+      double uf = us * wv;
+      if (a.do_peror) {   // scaled u and rhs for jcg_peror_kernel; the records are done with
+        a.u1[i] = us;
+        ((double *)a.p0)[2 * (size_t)a.nslices * kSlice + i] = a.rhs[i];
+      }
       a.u[i] = uf;
       a.rhs[i] = a.rhs[i] * (1.0 / wv);
       if (a.eta_update) {
