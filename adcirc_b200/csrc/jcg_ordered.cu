@@ -166,14 +166,14 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
   }
   __syncthreads();
 
-  double gprev = 0.0;                 // the eigenvalue estimate's last step
+  const double ztol = scalar_block && warp == 0 ? zbrent_tol(L.zeta) : 0.0;
   // chgcon for iteration `in` in the scalar block's first warp, from the
   // scalars the last exchange left in L.
   auto estimate = [&](int in) {
     if (warp != 0) return;
     double cme = L.cme, cmold = L.cmold;
     int adapt = L.adapt, ier = L.chg_ier;
-    if (adapt) chgcon_warp(L.gamma, L.rho, L.gamold, L.rhoold, L.zeta, tri, in, cme, cmold, gprev, adapt, ier);
+    if (adapt) chgcon_warp(L.gamma, L.rho, L.gamold, L.rhoold, L.zeta, ztol, a.itmax, tri, in, cme, cmold, adapt, ier);
     __syncwarp();
     if (lane == 0) {
       L.cme = cme;

@@ -954,7 +954,8 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       need_u = s_rec.need_u;
     }
   } else {
-    double cmold = a.itp->cmold, cme = a.itp->cme, gprev = 0.0;
+    double cmold = a.itp->cmold, cme = a.itp->cme;
+    const double ztol = zbrent_tol(zeta);
     int adapt = a.run_init ? 1 : a.itp->adapt, chg_ier = 0;
     for (int in = 0;; ++in) {
       const long long tw = clock64();
@@ -966,7 +967,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       if (s_hist < in || (in > 0 && s_done != 0)) break;
       if (adapt) {
         const double2 h = hist[max(in - 1, 0)], o = hist[max(in - 2, 0)];
-        chgcon_warp(h.x, h.y, o.x, o.y, zeta, tri, in, cme, cmold, gprev, adapt, chg_ier);
+        chgcon_warp(h.x, h.y, o.x, o.y, zeta, ztol, a.itmax, tri, in, cme, cmold, adapt, chg_ier);
       }
       if (lane == 0) {
         s_cme = cme;
