@@ -226,6 +226,7 @@ def load():
         "adc_kernel_times": (C.c_int, [vp, dp_, C.c_int]),
         "adc_set_jcg_blocks": (C.c_int, [vp, C.c_int]),
         "adc_jcg_layout": (C.c_int, [vp, ip_, ip_]),
+        "adc_set_wait_cycles": (C.c_int, [vp, C.c_longlong]),
         "adc_ensemble_create": (C.c_int, [C.c_int, C.POINTER(vp), C.POINTER(vp)]),
         "adc_ensemble_run": (C.c_int, [vp, C.c_int, C.POINTER(AdcStep), ip_, C.POINTER(AdcStepOut)]),
         "adc_ensemble_last_ms": (C.c_double, [vp]),

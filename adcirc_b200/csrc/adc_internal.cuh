@@ -23,6 +23,9 @@ constexpr int kSlice = 32;            // rows per SELL slice (one warp)
 constexpr int kGatherChunk = 8;       // per-node gathers issued together
 constexpr int kThreads = 256;
 constexpr long long kSpinCycles = 4000000000LL;  // ~2 s at 1.9 GHz
+// What a block whose wait has expired gives its copies and incoming stores in
+// flight (they take a microsecond or two) before it leaves: 0.1 ms.
+constexpr long long kDrainCycles = 200000;
 
 // Device-visible scalar state of the step and of ITPACK.
 struct Flags {
@@ -207,6 +210,7 @@ struct adc_ctx {
   int jcg_res_k, jcg_rows_max, jcg_halo_max, jcg_stage_bytes;
   int jr_o[9];                 // its shared-memory offsets
   size_t jcg_smem;
+  long long spin_cycles;       // limit of a wait inside a solve, 0: kSpinCycles
   int jcg_stage_wcap;
   unsigned char *jtab;         // one allocation behind the tables below
   unsigned char *jtab_room;    // the caller's room for them, if it has any

@@ -21,6 +21,8 @@ struct JcgArgs {
   Bar *bar;
   void *arrive;             // the barrier lines (see the kernels)
   Flags *flags;
+  long long spin;           // cycles a wait may take ...
+  unsigned spin_every;      // ... and polls between looks at the clock and the timeout flag
   int eta_update;
   int do_peror;
   int run_init;               // echall's per-solve initialisation inside the kernel

@@ -64,10 +64,9 @@ __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" 
 // itself): with one load per word, and the timeout flag read beside them, the
 // 296 x 296 polls of a barrier took 10,200 cycles of an iteration's 16,700 at
 // 100k rows (200 mixed-mode steps 58.5 -> 50.7 ms with this).  Bounded: the
-// limit and the flag are looked at once in 64 polls.
+// limit and the flag are looked at once in spin_every polls.
 template <int N>
-__device__ inline bool poll_full(volatile unsigned long long *p, unsigned long long (&v)[N],
-                          Flags *flags) {
+__device__ inline bool poll_full(volatile unsigned long long *p, unsigned long long (&v)[N], const JcgArgs &a) {
   const long long t0 = clock64();
   for (unsigned m = 1;; ++m) {
     bool full = true;
@@ -82,10 +81,10 @@ __device__ inline bool poll_full(volatile unsigned long long *p, unsigned long l
       full = full && (v[k] != kEmpty);
     }
     if (full) return true;
-    if (m % 64 != 0) continue;
-    if (*(volatile int *)&flags->timeout) return false;
-    if (clock64() - t0 > kSpinCycles) {
-      atomicExch(&flags->timeout, 1);
+    if ((m & (a.spin_every - 1)) != 0) continue;
+    if (*(volatile int *)&a.flags->timeout) return false;
+    if (clock64() - t0 > a.spin) {
+      atomicExch(&a.flags->timeout, 1);
       return false;
     }
   }
@@ -214,7 +213,7 @@ __device__ inline bool grid_phase(const JcgArgs &a, bool scalar_block, unsigned 
   for (int b = threadIdx.x; b <= a.nrb; b += blockDim.x) {
     volatile unsigned long long *ap = ((ArriveLine *)a.arrive + b)->slot[sl];
     unsigned long long v[3];
-    if (!poll_full<3>(ap, v, a.flags)) {
+    if (!poll_full<3>(ap, v, a)) {
       bad = 1;
       break;
     }

@@ -43,6 +43,7 @@ struct SlicePipe {
   int stage_bytes, s0, s1, first, step, lane;
   uint32_t parbits;
   int wcap;                   // slices wider than this are not staged
+  long long spin;             // cycles a wait may take
 
   __device__ bool staged(int sl) const { return meta[sl - s0].y <= wcap; }
 
@@ -69,23 +70,28 @@ struct SlicePipe {
     if (first < s1) issue(first, 0, vals);
     if (first + step < s1) issue(first + step, 1, vals);
   }
+  // Waits for a copy in flight for kDrainCycles more.
+  __device__ void drain(int st) {
+    const long long tw = clock64();
+    while (!mbar_try_wait(bar0 + st, (parbits >> st) & 1u) && clock64() - tw < kDrainCycles) {
+    }
+  }
+  // The answer is the warp's: lanes that look at the clock one by one may
+  // differ.
   __device__ bool wait(int st, bool other_in_flight) {
-    long long tw = clock64();
-    while (!mbar_try_wait(bar0 + st, (parbits >> st) & 1u)) {
-      if (clock64() - tw > kSpinCycles) {
-        if (lane == 0) {
-          atomicExch(&flags->timeout, 1);
-          // let the copy already issued into the other buffer land
-          if (other_in_flight) {
-            long long t1w = clock64();
-            while (!mbar_try_wait(bar0 + (st ^ 1), (parbits >> (st ^ 1)) & 1u) &&
-                   clock64() - t1w < kSpinCycles) {
-            }
-          }
-        }
-        __syncwarp();
-        return false;
+    const long long tw = clock64();
+    bool ok;
+    while (!(ok = mbar_try_wait(bar0 + st, (parbits >> st) & 1u)) && clock64() - tw <= spin) {
+    }
+    if (!__all_sync(0xffffffffu, ok)) {
+      if (lane == 0) {
+        atomicExch(&flags->timeout, 1);
+        // let this copy and the one already issued into the other buffer land
+        drain(st);
+        if (other_in_flight) drain(st ^ 1);
       }
+      __syncwarp();
+      return false;
     }
     parbits ^= 1u << st;
     return true;
@@ -143,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
   unsigned char *S_stage = (unsigned char *)(S_bar + 16);
   const int nhalo = !scalar_block ? a.halo_ptr[blockIdx.x + 1] - a.halo_ptr[blockIdx.x] : 0;
   SlicePipe pipe{S_stage + (size_t)(2 * warp) * a.stage_bytes, &S_bar[2 * warp], S_meta, a.lcol,
-                 a.flags, a.stage_bytes, s0, s1, s0 + warp, nwarps, lane, 0u, a.stage_wcap};
+                 a.flags, a.stage_bytes, s0, s1, s0 + warp, nwarps, lane, 0u, a.stage_wcap, a.spin};
   __shared__ ItpLocal L;              // used by the scalar block's thread 0 only
   __shared__ Rec s_rec;               // the record of the last reducing barrier
   unsigned gen = a.bar->gen;          // barrier generation, going on from solve to solve

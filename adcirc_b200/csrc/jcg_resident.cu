@@ -509,14 +509,17 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
     s_rem &= s_rem - 1u;
     if (s_rem == 0u) s_rem = smask;
   };
-  auto land = [&]() -> int {   // waits for the oldest copy in flight: its buffer
+  // waits for the oldest copy in flight: its buffer (kDrainCycles more when
+  // the wait has expired, so that no copy outlives the block)
+  auto land = [&]() -> int {
     const int st = (int)(l_cnt & 1u);
     const long long tw = clock64();
     while (!mbar_try_wait(&S_bar[2 * warp + st], (bar_par >> st) & 1u)) {
-      if (clock64() - tw > kSpinCycles) {
+      const long long dt = clock64() - tw;
+      if (dt > a.spin) {
         if (lane == 0) atomicExch(&a.flags->timeout, 1);
         bad = 1;
-        break;
+        if (dt > a.spin + kDrainCycles) break;
       }
     }
     bar_par ^= 1u << st;
@@ -555,8 +558,8 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       unsigned polls = 0;
       do {
         q = ld_w2(p);
-        if (q.y != g && ++polls % 64 == 0 &&
-            (clock64() - tw > kSpinCycles || *(volatile int *)&a.flags->timeout)) {
+        if (q.y != g && (++polls & (a.spin_every - 1)) == 0 &&
+            (clock64() - tw > a.spin || *(volatile int *)&a.flags->timeout)) {
           atomicExch(&a.flags->timeout, 1);
           bad = 1;
           break;
@@ -591,6 +594,8 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
   __syncthreads();
 
   int m = 0;
+  bool ended = false;             // the solve has ended, without an expired wait in this block
+  unsigned e = 0;                 // exchanges so far: parity of the double buffers
   if (row_warp) {
 #pragma unroll
     for (int k = 0; k < K; ++k) dp[k] = 0.0;
@@ -598,7 +603,6 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
     for (int k = 0; k < KU; ++k) up[k] = 0.0;
     double c1 = 0.0, c2 = 0.0, c3 = 0.0, c4 = 0.0;
     int need_u = !q1_in, halt = 0;
-    unsigned e = 0;                 // exchanges so far: parity of the double buffers
     W2 emptied = {0ull, 0ull};      // grid form: old word of the slot this lane emptied last
     W2 hq = {0ull, 0ull};           // the thread's first halo word, requested early
     for (;; ++m) {
@@ -781,7 +785,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
         if (m > 0 && !need_u) update_u();
         const long long tw = clock64();
         while (!mbar_try_wait_cluster(&s_xbar[e & 1], ((e - 1u) >> 1) & 1u)) {
-          if (clock64() - tw > kSpinCycles) {
+          if (clock64() - tw > a.spin) {
             atomicExch(&a.flags->timeout, 1);
             bad = 1;
             break;
@@ -818,7 +822,8 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
             for (unsigned polls = 1;; ++polls) {
               poll_slot(line, y.x, y.y, z.x);
               if (y.x != kEmpty && y.y != kEmpty && (!need_u || z.x != kEmpty)) break;
-              if (polls % 64 == 0 && (clock64() - tw > kSpinCycles || *(volatile int *)&a.flags->timeout)) {
+              if ((polls & (a.spin_every - 1)) == 0 &&
+                  (clock64() - tw > a.spin || *(volatile int *)&a.flags->timeout)) {
                 atomicExch(&a.flags->timeout, 1);
                 bad = 1;
                 break;
@@ -899,7 +904,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
                 sqd >= squd * (1.0 - low) * zeta)) {
             const long long tw = clock64();
             while (s_cme_m < m) {
-              if (clock64() - tw > kSpinCycles) {
+              if (clock64() - tw > a.spin) {
                 if (lane == 0) atomicExch(&a.flags->timeout, 1);
                 bad = 1;
                 break;
@@ -938,7 +943,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
           s_done = failed ? 2 : 1;
         }
         while (l_cnt != s_cnt) land();   // the copies in flight
-        if (failed) return;
+        ended = !failed;
         break;
       }
       if (tid == 0) {
@@ -960,7 +965,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
     for (int in = 0;; ++in) {
       const long long tw = clock64();
       while (s_hist < in && s_done == 0) {
-        if (clock64() - tw > 2 * kSpinCycles) break;   // the row warps have given up before
+        if (clock64() - tw > 2 * a.spin) break;   // the row warps have given up before
       }
       __syncwarp();
       __threadfence_block();
@@ -976,10 +981,10 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       }
       __syncwarp();
     }
-    if (s_done != 1) return;
+    ended = s_done == 1;
     __threadfence_block();
     m = s_m;
-    if (b == 0 && lane == 0) {
+    if (ended && b == 0 && lane == 0) {
       const Scal s = sc;
       const int halt = s_rec.halt;
       const double stptst = s.tl / s.tr;
@@ -1005,7 +1010,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
   // ---- epilogue: unscal (itpackv.F:2447-2477), the GWCE eta update
   // (gwce.F:2006-2008) and wet/dry pass D1, which took a launch of 2 us and a
   // second pass over ETA2 and NODECODE by itself
-  if (row_warp) {
+  if (row_warp && ended) {
     double wv[K], e1[K], uf[K], dp[K];
     int nc[K];
 #pragma unroll
@@ -1042,12 +1047,26 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       }
     }
   }
-  if (kGrid && b == 0 && tid == 0) {
+  if (kGrid && ended && b == 0 && tid == 0) {
     a.bar->count = ag;
     a.bar->gen = tag;
   }
   __syncwarp();
-  if (!kGrid) cluster_barrier();   // no block leaves while another may read its shared memory
+  if (!kGrid) {
+    // No block leaves while another may read its shared memory or store into
+    // it, after an expired wait either: by the barrier every block has issued
+    // its last stores (each of its waits is bounded), and they get time to
+    // come in, those of the exchange that this block did not complete and
+    // those of the next, which a block that did may have begun.
+    cluster_barrier();
+    if (row_warp && !ended) {
+      const long long tw = clock64();
+      while (!(mbar_try_wait_cluster(&s_xbar[e & 1], ((e - 1u) >> 1) & 1u) &&
+               mbar_try_wait_cluster(&s_xbar[(e + 1u) & 1], (e >> 1) & 1u)) &&
+             clock64() - tw < kDrainCycles) {
+      }
+    }
+  }
 #undef LE
 }
 

@@ -889,6 +889,13 @@ int adc_set_jcg_blocks(adc_ctx *c, int nrb) {
   return ADC_OK;
 }
 
+int adc_set_wait_cycles(adc_ctx *c, long long cycles) {
+  if (!c || cycles < 0) return ADC_ERR_ARG;
+  drop_graphs(c);   // the limit is a launch argument
+  c->spin_cycles = cycles;
+  return ADC_OK;
+}
+
 int adc_jcg_layout(adc_ctx *c, int *row_blocks, int *resident) {
   if (!c) return ADC_ERR_ARG;
   if (row_blocks) *row_blocks = c->jcg_rows_blocks;

@@ -632,6 +632,12 @@ int adc_kernel_times(adc_ctx *ctx, double *ms, int n);
 int adc_set_jcg_blocks(adc_ctx *ctx, int row_blocks);
 int adc_jcg_layout(adc_ctx *ctx, int *row_blocks, int *resident);
 
+/* SM clock cycles that a wait inside the context's solver (for another block
+ * or a copy) may take before the solve gives up and the call returns
+ * ADC_ERR_TIMEOUT; 0 restores the default of 4e9, about 2 s.  No reference
+ * counterpart. */
+int adc_set_wait_cycles(adc_ctx *ctx, long long cycles);
+
 /* Ensembles (no reference counterpart; the reference runs one mesh per
  * process, adcirc.F:475-476): n independent bound contexts stepped
  * together.  Every replayed time step is one captured CUDA graph holding
