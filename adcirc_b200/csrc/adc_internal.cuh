@@ -277,6 +277,7 @@ int launch_shift_friction(adc_ctx *c, bool whole);
 int launch_gwce(adc_ctx *c);
 int launch_jcg(adc_ctx *c, int eta_update, bool d1);
 void jcg_clear_barrier(adc_ctx *c);
+int jcg_reset_exchange(adc_ctx *c);
 int launch_wetdry(adc_ctx *c, bool whole, bool d1_done);
 int launch_momentum(adc_ctx *c, bool whole, int *log);
 

@@ -178,6 +178,8 @@ extern "C" int adc_hotstart_read(adc_ctx *c, const char *path) {
   }
   std::fclose(f);
   c->met_pending = 0;
+  // the file's flags end a timeout: nothing of a failed solve may stay
+  if (int rc = jcg_reset_exchange(c)) return rc;
   // the cached GWCE element entries describe the old state: rebuild in full
   {
     int *w = (int *)(c->flags + 1);

@@ -630,6 +630,18 @@ void jcg_clear_barrier(adc_ctx *c) {
   c->launches++;
 }
 
+// Empties all that the solver's blocks have exchanged: for a new layout, and
+// after a solve that gave up, which leaves posts of generations that the next
+// solve would take for its own.
+int jcg_reset_exchange(adc_ctx *c) {
+  jcg_clear_barrier(c);
+  const size_t bytes = (size_t)c->nslices * kSlice * sizeof(double4);
+  ADC_CUDA(cudaMemsetAsync(c->jp[0], 0, bytes, c->stream));
+  ADC_CUDA(cudaMemsetAsync(c->jp[1], 0, bytes, c->stream));
+  ADC_CUDA(cudaStreamSynchronize(c->stream));
+  return ADC_OK;
+}
+
 int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int defer_drift, int d1) {
   JcgArgs a;
   a.do_peror = do_peror;

@@ -881,12 +881,7 @@ int adc_set_jcg_blocks(adc_ctx *c, int nrb) {
   const JcgHostSell hs{sl_ptr.data(), sl_w.data(), col.data(), rlen.data()};
   TRY(jcg_setup_grid(c, &hs));
   TRY(dalloc((char **)&c->jlines, 2 * 128 * (size_t)c->jcg_rows_blocks));
-  jcg_clear_barrier(c);
-  // no exchange word of the old layout may pass for one of the new
-  ADC_CUDA(cudaMemsetAsync(c->jp[0], 0, nsl * kSlice * sizeof(double4), c->stream));
-  ADC_CUDA(cudaMemsetAsync(c->jp[1], 0, nsl * kSlice * sizeof(double4), c->stream));
-  ADC_CUDA(cudaStreamSynchronize(c->stream));
-  return ADC_OK;
+  return jcg_reset_exchange(c);   // no exchange word of the old layout may pass for one of the new
 }
 
 int adc_set_wait_cycles(adc_ctx *c, long long cycles) {

@@ -51,3 +51,28 @@ def test_expired_wait_is_an_error(lib, form):
     its2, got = _run(_case(nx, ny), prec, 6)
     assert np.array_equal(its, its2)
     assert all(np.array_equal(want[k], got[k]) for k in want)
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_hotstart_resumes_after_an_expired_wait(lib, tmp_path, form):
+    """A dump taken before, read back into the same context: the run goes on
+    bit for bit, whatever the failed solve had exchanged."""
+    from adcirc_b200 import model
+    nx, ny, prec = FORMS[form]
+    its, want = _run(_case(nx, ny), prec, 8)
+    case = _case(nx, ny)
+    gpu = model.GpuModel(case, prec)
+    got = list(gpu.run(1, 4)[0])
+    gpu.hotstart_write(tmp_path / "hs")
+    assert lib.adc_set_wait_cycles(gpu.h, 1) == 0
+    for _ in range(3):
+        with pytest.raises(model.AdcError, match="status -5"):
+            gpu.step(5)
+    assert lib.adc_set_wait_cycles(gpu.h, 0) == 0
+    gpu.hotstart_read(tmp_path / "hs")
+    got += list(gpu.run(5, 4)[0])
+    gpu.sync_to_host()
+    gpu.close()
+    assert np.array_equal(its, got)
+    bad = [k for k in want if not np.array_equal(want[k], case.arrays[k])]
+    assert not bad, bad
