@@ -962,14 +962,23 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
     double cmold = a.itp->cmold, cme = a.itp->cme;
     const double ztol = zbrent_tol(zeta);
     int adapt = a.run_init ? 1 : a.itp->adapt, chg_ier = 0;
+    // What the row warps have left in shared memory is read by lane 0 alone:
+    // lanes that read it one by one may differ, and all of them go on together.
+    int done = 0;   // s_done, where lane 0 last read it
     for (int in = 0;; ++in) {
-      const long long tw = clock64();
-      while (s_hist < in && s_done == 0) {
-        if (clock64() - tw > 2 * a.spin) break;   // the row warps have given up before
+      int go = 0;
+      if (lane == 0) {
+        const long long tw = clock64();
+        while (s_hist < in && s_done == 0) {
+          if (clock64() - tw > 2 * a.spin) break;   // the row warps have given up before
+        }
+        done = s_done;
+        go = s_hist >= in && (in == 0 || done == 0);
+        __threadfence_block();
       }
-      __syncwarp();
-      __threadfence_block();
-      if (s_hist < in || (in > 0 && s_done != 0)) break;
+      go = __shfl_sync(0xffffffffu, go, 0);
+      __syncwarp();   // lane 0's reads before every lane's
+      if (!go) break;
       if (adapt) {
         const double2 h = hist[max(in - 1, 0)], o = hist[max(in - 2, 0)];
         chgcon_warp(h.x, h.y, o.x, o.y, zeta, ztol, a.itmax, tri, in, cme, cmold, adapt, chg_ier);
@@ -981,8 +990,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       }
       __syncwarp();
     }
-    ended = s_done == 1;
-    __threadfence_block();
+    ended = __shfl_sync(0xffffffffu, done, 0) == 1;
     m = s_m;
     if (ended && b == 0 && lane == 0) {
       const Scal s = sc;
