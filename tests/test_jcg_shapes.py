@@ -110,3 +110,54 @@ def test_tight_shapes_solve(lib, n, near, lo, hi, far, itmax):
     assert (ie, it) == (ie2, it2)
     assert np.abs(u - u2).max() <= 1e-9 * np.abs(u2).max()
     assert np.abs(c - c2).max() <= 1e-14 * np.abs(c2).max()
+
+
+@pytest.mark.gpu
+def test_staged_slices_of_uneven_width(lib):
+    """Blocks of 4,320 rows (nine slices a warp, most of them streamed).  In
+    each, a warp's first slice has rows of 12 neighbours, the last of them the
+    block's row 4,094 or 4,095, whose column word 0x7ff0 or 0x7ff8 is the top
+    of a double that is no number; the third has rows of one neighbour, so
+    that its buffer still holds words of the first past its own end."""
+    import oracle
+    from adcirc_b200._lib import dp_, ip_, ptr
+    orc = oracle.load()
+    per = 15 * 9 * 32
+    n = SMS * per
+    i = np.arange(n)
+    local = i % per
+    k = local // 32 // 15
+    cols = np.zeros((n, 12), np.int64)
+    use = np.zeros((n, 12), bool)
+    for q in range(11):
+        cols[:, q] = i ^ (q + 1)
+        use[:, q] = (k == 0) | (q == 0) | ((q == 1) & (k != 2))
+    cols[:, 11] = i - local + 4094 + i % 2
+    use[:, 11] = k == 0
+    v = np.where(use, 0.05 + 0.3 * ((np.minimum(cols, i[:, None]) * 7919) % 1009) / 1009.0, 0.0)
+    v[:, 11] *= 1e-6
+    rng = np.random.default_rng(12)
+    jcoef = np.zeros((n, 13), np.int32, order="F")
+    coef = np.zeros((n, 13), order="F")
+    jcoef[:, 0] = i + 1
+    coef[:, 0] = 0.5 + np.abs(v).sum(1) * rng.uniform(1.05, 1.3, n)
+    jcoef[:, 1:] = np.where(use, cols + 1, 0)
+    coef[:, 1:] = v
+    rhs, u0 = rng.standard_normal(n), 1e-2 * rng.standard_normal(n)
+    got = []
+    for jcg, dfault, reset in ((lib.adc_jcg, lib.adc_dfault, lib.adc_jcg_reset),
+                               (orc.orc_jcg, orc.orc_dfault, orc.orc_itpack_reset)):
+        reset()
+        j, c, r, u = jcoef.copy(order="F"), coef.copy(order="F"), rhs.copy(), u0.copy()
+        iparm, rparm = np.zeros(12, np.int32), np.zeros(12)
+        dfault(ptr(iparm, ip_), ptr(rparm, dp_))
+        iparm[0], rparm[0] = 200, 1e-8
+        nw = 4 * n + 800
+        wksp, iwksp, ier = np.zeros(nw), np.zeros(3 * n, np.int32), C.c_int(-1)
+        jcg(C.byref(C.c_int(n)), C.byref(C.c_int(n)), C.byref(C.c_int(13)), ptr(j, ip_), ptr(c, dp_),
+            ptr(r, dp_), ptr(u, dp_), ptr(iwksp, ip_), C.byref(C.c_int(nw)), ptr(wksp, dp_),
+            ptr(iparm, ip_), ptr(rparm, dp_), C.byref(ier))
+        got.append((ier.value, int(iparm[0]), u))
+    (ie, it, u), (ie2, it2, u2) = got
+    assert (ie, it) == (ie2, it2)
+    assert np.abs(u - u2).max() <= 1e-9 * np.abs(u2).max()
