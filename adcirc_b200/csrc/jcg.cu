@@ -36,7 +36,6 @@
 #include <cstring>
 #include <vector>
 #include <algorithm>
-#include <mutex>
 
 namespace adc {
 
@@ -549,30 +548,17 @@ namespace adc {
 // one context's need: contexts with different layouts (the members of an
 // ensemble) then all launch.
 //
-// The limit is also what a launch may ask for (`limit`).  It is set once per
-// kernel and device.
+// The limit is also what a launch may ask for (`limit`).  It belongs to the
+// device's context, which a host program may reset, so it is set for every
+// layout.
 int jcg_smem_limit(const void *fn, size_t *limit) {
-  struct Known {
-    const void *fn;
-    int dev;
-    size_t bytes;
-  };
-  static std::mutex mu;
-  static std::vector<Known> known;
   int dev = 0, optin = 0;
   ADC_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  for (const Known &k : known)
-    if (k.fn == fn && k.dev == dev) {
-      if (limit) *limit = k.bytes;
-      return ADC_OK;
-    }
   ADC_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   cudaFuncAttributes fa;
   ADC_CUDA(cudaFuncGetAttributes(&fa, fn));
   const size_t bytes = (size_t)optin - fa.sharedSizeBytes;
   ADC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  known.push_back({fn, dev, bytes});
   if (limit) *limit = bytes;
   return ADC_OK;
 }

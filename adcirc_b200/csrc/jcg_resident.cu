@@ -58,7 +58,6 @@
 #include <cstring>
 #include <vector>
 #include <algorithm>
-#include <mutex>
 
 namespace adc {
 
@@ -1183,22 +1182,8 @@ static size_t align_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 
 static int block_begin(int nslices, int nrb, int b) { return (int)((long long)nslices * b / nrb); }
 
-// Whether one cluster of 16 blocks of `fn` can run; asked once per kernel and
-// device, at the shared-memory need of the first caller or more.
+// Whether one cluster of 16 blocks of `fn` can run.
 static bool cluster16(const void *fn, size_t smem) {
-  struct Known {
-    const void *fn;
-    int dev;
-    size_t bytes;
-    bool ok;
-  };
-  static std::mutex mu;
-  static std::vector<Known> known;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  std::lock_guard<std::mutex> lock(mu);
-  for (const Known &k : known)
-    if (k.fn == fn && k.dev == dev && (k.ok ? smem <= k.bytes : smem >= k.bytes)) return k.ok;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = 16;
   cfg.blockDim = kResThreads;
@@ -1213,7 +1198,6 @@ static bool cluster16(const void *fn, size_t smem) {
   const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                   cudaOccupancyMaxActiveClusters(&nc, fn, &cfg) == cudaSuccess && nc >= 1;
   if (!ok) cudaGetLastError();
-  known.push_back({fn, dev, smem, ok});
   return ok;
 }
 
