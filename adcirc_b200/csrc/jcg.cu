@@ -654,7 +654,7 @@ int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int 
   a.arrive = c->jlines;
   a.flags = c->flags;
   a.spin = c->spin_cycles > 0 ? c->spin_cycles : kSpinCycles;
-  a.spin_every = a.spin < 1000000 ? 1 : 64;   // 64 polls may take 100,000 cycles
+  a.spin_mask = a.spin < 1000000 ? 0 : 63;   // 64 polls may take 100,000 cycles
   a.eta_update = eta_update;
   a.d1 = d1;
   a.nodecode = c->nodecode;

@@ -22,7 +22,7 @@ struct JcgArgs {
   void *arrive;             // the barrier lines (see the kernels)
   Flags *flags;
   long long spin;           // cycles a wait may take ...
-  unsigned spin_every;      // ... and polls between looks at the clock and the timeout flag
+  unsigned spin_mask;       // ... and polls between looks at the clock and the timeout flag, less one
   int eta_update;
   int do_peror;
   int run_init;               // echall's per-solve initialisation inside the kernel

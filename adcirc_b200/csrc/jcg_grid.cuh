@@ -64,7 +64,7 @@ __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" 
 // itself): with one load per word, and the timeout flag read beside them, the
 // 296 x 296 polls of a barrier took 10,200 cycles of an iteration's 16,700 at
 // 100k rows (200 mixed-mode steps 58.5 -> 50.7 ms with this).  Bounded: the
-// limit and the flag are looked at once in spin_every polls.
+// limit and the flag are looked at once in spin_mask + 1 polls.
 template <int N>
 __device__ inline bool poll_full(volatile unsigned long long *p, unsigned long long (&v)[N], const JcgArgs &a) {
   const long long t0 = clock64();
@@ -81,7 +81,7 @@ __device__ inline bool poll_full(volatile unsigned long long *p, unsigned long l
       full = full && (v[k] != kEmpty);
     }
     if (full) return true;
-    if ((m & (a.spin_every - 1)) != 0) continue;
+    if ((m & a.spin_mask) != 0) continue;
     if (*(volatile int *)&a.flags->timeout) return false;
     if (clock64() - t0 > a.spin) {
       atomicExch(&a.flags->timeout, 1);

@@ -230,13 +230,13 @@ __device__ __forceinline__ void sub4(double &acc, const double (&v)[4], const do
   for (int q = 0; q < 4; ++q) acc = acc - v[q] * xx[q];
 }
 
-// Two slices (shared memory) with columns at p0 and p1 and values o0 and o1
-// bytes after, side by side: their two chains of sums overlap.
-__device__ __forceinline__ void pair_spmv(double &acc0, double &acc1, const unsigned char *p0, int o0, int ng0,
-                                          const unsigned char *p1, int o1, int ng1, const unsigned char *x) {
+// Two slices at p0 and p1 (shared memory) side by side: their two chains of
+// sums overlap.
+__device__ __forceinline__ void pair_spmv(double &acc0, double &acc1, const unsigned char *p0, int ng0,
+                                          const unsigned char *p1, int ng1, const unsigned char *x) {
   const int lane = threadIdx.x & 31;
   const uint4 c0 = ((const uint4 *)p0)[lane], c1 = ((const uint4 *)p1)[lane];
-  const double *v0 = (const double *)(p0 + o0) + lane, *v1 = (const double *)(p1 + o1) + lane;
+  const double *v0 = (const double *)(p0 + ng0 * 512) + lane, *v1 = (const double *)(p1 + ng1 * 512) + lane;
   {
     double a[4], b[4], xa[4], xb[4];
     load4<0>(a, xa, c0, v0, x);
@@ -491,10 +491,6 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
   }
   unsigned s_rem = smask;            // the slices still to copy in this round
   unsigned s_cnt = 0u, l_cnt = 0u;   // copies issued, copies landed
-  // A buffer holds the values, then the columns, each in room for the widest
-  // staged slice: slots past a slice's end multiply what is there by zero, and
-  // a column word of another slice may read as no number.
-  const int s_col = a.stage_bytes / 5 * 4;   // 2,048 of 2,560 bytes a group
   auto issue = [&]() {   // copies the next streamed slice into its buffer
     const int k = __ffs(s_rem) - 1;
     if (lane == 0) {
@@ -505,8 +501,8 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       uint64_t *const bar = &S_bar[2 * warp + st];
       unsigned char *const dst = stage + st * a.stage_bytes;
       mbar_expect_tx(bar, cb + vb);
-      bulk_load(dst + s_col, a.rcol + (size_t)mt.z * 32, cb, bar);
-      if (vb) bulk_load(dst, a.soff + mt.x, vb, bar);
+      bulk_load(dst, a.rcol + (size_t)mt.z * 32, cb, bar);
+      if (vb) bulk_load(dst + cb, a.soff + mt.x, vb, bar);
     }
     ++s_cnt;
     s_rem &= s_rem - 1u;
@@ -518,11 +514,10 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
     const int st = (int)(l_cnt & 1u);
     const long long tw = clock64();
     while (!mbar_try_wait(&S_bar[2 * warp + st], (bar_par >> st) & 1u)) {
-      const long long dt = clock64() - tw;
-      if (dt > a.spin) {
+      if (clock64() - tw > a.spin) {
         if (lane == 0) atomicExch(&a.flags->timeout, 1);
         bad = 1;
-        if (dt > a.spin + kDrainCycles) break;
+        if (clock64() - tw - kDrainCycles > a.spin) break;
       }
     }
     bar_par ^= 1u << st;
@@ -530,7 +525,8 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
     return st;
   };
   if (smask) {
-    // numbers from the start
+    // slots past a slice's end multiply what the buffer holds by zero: it
+    // must hold numbers (see staged_values)
     for (int q = lane; q < 2 * a.stage_bytes / 16; q += 32) ((uint4 *)stage)[q] = make_uint4(0u, 0u, 0u, 0u);
     fence_proxy_async_all();
     __syncwarp();
@@ -560,7 +556,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       unsigned polls = 0;
       do {
         q = ld_w2(p);
-        if (q.y != g && (++polls & (a.spin_every - 1)) == 0 &&
+        if (q.y != g && (++polls & a.spin_mask) == 0 &&
             (clock64() - tw > a.spin || *(volatile int *)&a.flags->timeout)) {
           atomicExch(&a.flags->timeout, 1);
           bad = 1;
@@ -710,27 +706,10 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
             double a0 = 0.0, a1 = 0.0;
             if (in0 || in1) {
               const unsigned char *p0 = stage, *p1 = stage;
+              if (in0) p0 = m0.w >= 0 ? sm + a.o_res + m0.w : stage + land() * a.stage_bytes;
+              if (in1) p1 = m1.w >= 0 ? sm + a.o_res + m1.w : stage + land() * a.stage_bytes;
               const int g0 = slot_groups((in0 ? m0 : m1).y), g1 = slot_groups((in1 ? m1 : m0).y);
-              int o0 = g0 * 512, o1 = g1 * 512;   // a resident slice: columns, then values
-              if (in0) {
-                if (m0.w >= 0) {
-                  p0 = sm + a.o_res + m0.w;
-                } else {
-                  p0 = stage + land() * a.stage_bytes + s_col;
-                  o0 = -s_col;
-                }
-              }
-              if (in1) {
-                if (m1.w >= 0) {
-                  p1 = sm + a.o_res + m1.w;
-                } else {
-                  p1 = stage + land() * a.stage_bytes + s_col;
-                  o1 = -s_col;
-                }
-              }
-              if (!in0) p0 = p1, o0 = o1;
-              if (!in1) p1 = p0, o1 = o0;
-              pair_spmv(a0, a1, p0, o0, g0, p1, o1, g1, xd);
+              pair_spmv(a0, a1, in0 ? p0 : p1, g0, in1 ? p1 : p0, g1, xd);
             }
             if (m0.w == -1 || (has1 && m1.w == -1)) {
               __syncwarp();
@@ -841,7 +820,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
             for (unsigned polls = 1;; ++polls) {
               poll_slot(line, y.x, y.y, z.x);
               if (y.x != kEmpty && y.y != kEmpty && (!need_u || z.x != kEmpty)) break;
-              if ((polls & (a.spin_every - 1)) == 0 &&
+              if ((polls & a.spin_mask) == 0 &&
                   (clock64() - tw > a.spin || *(volatile int *)&a.flags->timeout)) {
                 atomicExch(&a.flags->timeout, 1);
                 bad = 1;
@@ -1224,6 +1203,13 @@ static int res_k(int k, bool grid) {
 // the planner has left it: kRegs' groups beyond the first.
 static bool reads_resident(int k, int w) { return k <= 2 && slot_groups(w) > 1; }
 
+// Whether behind a staged slice of width w a buffer of `groups` groups holds
+// values only.  A buffer has a slice's columns and, behind them, its values,
+// and slots past its end multiply what is there by zero: with slices of no or
+// one slot beside others of two groups that would be column words, which may
+// read as no number.  Such slices are read in place.
+static bool staged_values(int w, int groups) { return 512 * slot_groups(w) + 256 * w >= 512 * groups; }
+
 // Fills `p` for a matrix of n rows, on the host alone: `limit(k, grid, bytes)`
 // gives the dynamic shared memory an instance may use, `cluster(k, bytes)`
 // whether 16 of its blocks can be a cluster.  done = false where the resident
@@ -1382,7 +1368,7 @@ static int resident_shape(int n, const JcgHostSell *h, int itmax, int nrb_req, i
               if (used + sz <= room) {
                 meta[s0 + ls].w = (int)used;
                 used += sz;
-              } else if (sz > stage) {
+              } else if (sz > stage || !staged_values(h->sl_w[s0 + ls], (int)(stage / slice_bytes(1)))) {
                 meta[s0 + ls].w = -2;
               }
             }
