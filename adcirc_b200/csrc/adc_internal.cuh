@@ -26,6 +26,7 @@ constexpr long long kSpinCycles = 4000000000LL;  // ~2 s at 1.9 GHz
 // What a block whose wait has expired gives its copies and incoming stores in
 // flight (they take a microsecond or two) before it leaves: 0.1 ms.
 constexpr long long kDrainCycles = 200000;
+constexpr size_t kEstOffset = 128;    // flags, LHS words and tickets take 120 bytes
 
 // Device-visible scalar state of the step and of ITPACK.
 struct Flags {
@@ -58,6 +59,22 @@ struct Itp {
       stptst, cmold, srelpr, rparm1;
   Rec rec;
   double dtnrm, unorm;   // peror norms
+};
+
+// What a solve leaves for the estimate's last value, if its stopping test did
+// not need it: chgcon runs again over the recorded parcon coefficients
+// (gamma, rho), which follow, when a caller asks for it (jcg_estimate).
+struct alignas(16) EstRec {
+  double zeta, cme0, cmold0, sqd, squd;   // of the solve; sqrt(d.d) and sqrt(udnm) of its last test
+  int m, itmax, adapt0, exact;            // iterations; exact: nothing is left to do
+  int serial;                             // counts the solves that wrote this
+};
+
+// The estimate's last value and what chgcon and pstop left with it.
+struct Estimate {
+  double cme, cmold, stptst;
+  int adapt, ier;
+  int serial;   // of the solve (host: the last one formed)
 };
 
 struct Bar {
@@ -228,6 +245,8 @@ struct adc_ctx {
   int2 *jpush;
   // flags / steps
   adc::Flags *flags;
+  adc::Estimate est_last;   // host: as last formed, for several looks at one solve
+  adc::EstRec *est;      // 128 bytes behind the flags; then itmax + 2 pairs (gamma, rho)
   int *tickets;          // blocks done, of the kernels whose last block ends a pass
   adc_step_t *steps;     // device step table
   int steps_cap;
@@ -277,6 +296,9 @@ int launch_shift_friction(adc_ctx *c, bool whole);
 int launch_gwce(adc_ctx *c);
 int launch_jcg(adc_ctx *c, int eta_update, bool d1);
 void jcg_clear_barrier(adc_ctx *c);
+int jcg_estimate(const EstRec *est, cudaStream_t stream, Estimate &out, bool &have, const EstRec *head = nullptr,
+                 const double2 *pairs = nullptr, int npairs = 0);
+int read_state(adc_ctx *c, Flags &f, Estimate &est, bool &have);
 int jcg_reset_exchange(adc_ctx *c);
 int launch_wetdry(adc_ctx *c, bool whole, bool d1_done);
 int launch_momentum(adc_ctx *c, bool whole, int *log);

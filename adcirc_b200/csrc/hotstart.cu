@@ -99,6 +99,13 @@ extern "C" int adc_hotstart_write(adc_ctx *c, const char *path) {
   h.nrec = (int64_t)recs.size();
   bool ok = std::fwrite(&h, sizeof(h), 1, f) == 1;
   std::vector<char> buf;
+  Flags flags;
+  Estimate est;
+  bool have;
+  if (int rc = read_state(c, flags, est, have)) {
+    std::fclose(f);
+    return rc;
+  }
   for (const HsRec &r : recs) {
     if (!ok) break;
     char name[32];
@@ -109,6 +116,15 @@ extern "C" int adc_hotstart_write(adc_ctx *c, const char *path) {
     if (r.bytes > 0 && cudaMemcpy(buf.data(), r.dev, r.bytes, cudaMemcpyDeviceToHost) != cudaSuccess) {
       std::fclose(f);
       return cuda_fail(cudaGetLastError(), "adc_hotstart_write: device copy");
+    }
+    if (have && r.dev == c->flags) ((Flags *)buf.data())->cme = est.cme;
+    if (have && r.dev == c->itp) {
+      Itp *it = (Itp *)buf.data();
+      it->cme = est.cme;
+      it->cmold = est.cmold;
+      it->stptst = est.stptst;
+      it->adapt = est.adapt;
+      it->chg_ier = est.ier;
     }
     ok = std::fwrite(name, sizeof(name), 1, f) == 1 && std::fwrite(&nb, sizeof(nb), 1, f) == 1 &&
          (r.bytes == 0 || std::fwrite(buf.data(), r.bytes, 1, f) == 1);
@@ -178,6 +194,8 @@ extern "C" int adc_hotstart_read(adc_ctx *c, const char *path) {
   }
   std::fclose(f);
   c->met_pending = 0;
+  const int exact = 1;   // the file's estimate
+  ADC_CUDA(cudaMemcpy(&c->est->exact, &exact, sizeof(int), cudaMemcpyHostToDevice));
   // the file's flags end a timeout: nothing of a failed solve may stay
   if (int rc = jcg_reset_exchange(c)) return rc;
   // the cached GWCE element entries describe the old state: rebuild in full

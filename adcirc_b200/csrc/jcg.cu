@@ -39,165 +39,6 @@
 
 namespace adc {
 
-// ---------------------------------------------------------------- scalars
-// determ (itpackv.F:1029-1068): the three-term recurrence for
-// det(tri - x I), evaluated with the two trailing values in registers
-// (same operations, same order as the wk1/wk2 arrays of the reference).
-// tri(i,1) = t1[i-1], tri(i,2) = t2[i-1], held in shared memory.
-__device__ double determ_d(int n, const double *t1, const double *t2, double xlmda) {
-  double w2 = t1[n - 1] - xlmda;                       // wk2(n)
-  double w1 = (t1[n - 2] - xlmda) * w2 + t2[n - 1];    // wk2(n-1)
-  for (int l = n - 2; l >= 1; --l) {
-    double w = (t1[l - 1] - xlmda) * w1 + t2[l] * w2;  // wk2(l)
-    w2 = w1;
-    w1 = w;
-  }
-  return w1;
-}
-
-// zbrent (itpackv.F:2521-2781): Brent root of the characteristic
-// polynomial of the CG tridiagonal on [a, b].
-__device__ void zbrent_d(int n, const double *t1, const double *t2, double eps, double t,
-                         double &a, double &b, int &maxfn, int &ier) {
-  double c = 0, d = 0, e = 0, p, q, r, s, fa, fb, fc, tol, rm, rone, temp;
-  ier = 0;
-  int ic = 2;
-  fa = determ_d(n, t1, t2, a);
-  fb = determ_d(n, t1, t2, b);
-  s = b;
-  if ((fa > 0.0 && fb > 0.0) || (fa < 0.0 && fb < 0.0)) {
-    ier = 502;
-    maxfn = ic;
-    return;
-  }
-  bool reset = true;
-  for (;;) {
-    if (reset) {
-      c = a;
-      fc = fa;
-      d = b - c;
-      e = d;
-    }
-    reset = false;
-    if (!(fabs(fc) >= fabs(fb))) {
-      a = b; b = c; c = a;
-      fa = fb; fb = fc; fc = fa;
-    }
-    tol = t * fmax(fabs(b), 0.1);
-    rm = (c - b) * 0.5;
-    if (fabs(fb) <= eps || fabs(c - b) <= tol) {
-      a = c;
-      maxfn = ic;
-      return;
-    }
-    if (ic >= maxfn) {
-      ier = 501;
-      a = c;
-      maxfn = ic;
-      return;
-    }
-    bool bisect = false;
-    if (fabs(e) < tol || fabs(fa) <= fabs(fb)) {
-      bisect = true;
-    } else {
-      s = fb / fa;
-      if (a == c) {
-        p = (c - b) * s;
-        q = 1.0 - s;
-      } else {
-        q = fa / fc;
-        r = fb / fc;
-        rone = r - 1.0;
-        p = s * ((c - b) * q * (q - r) - (b - a) * rone);
-        q = (q - 1.0) * rone * (s - 1.0);
-      }
-      if (p > 0.0) q = -q;
-      if (p < 0.0) p = -p;
-      s = e;
-      e = d;
-      if (p + p >= 3.0 * rm * q || p + p >= fabs(s * q)) {
-        bisect = true;
-      } else {
-        d = p / q;
-      }
-    }
-    if (bisect) {
-      e = rm;
-      d = e;
-    }
-    a = b;
-    fa = fb;
-    temp = d;
-    if (fabs(temp) <= 0.5 * tol) temp = copysign(0.5 * tol, rm);
-    b = b + temp;
-    s = b;
-    fb = determ_d(n, t1, t2, s);
-    ic = ic + 1;
-    if (fb == 0.0 || fc == 0.0) continue;
-    if ((fb > 0.0 && fc < 0.0) || (fb < 0.0 && fc > 0.0)) continue;
-    reset = true;
-  }
-}
-
-// int(-log10(zeta)) as a glibc-linked Fortran build evaluates it: the
-// logarithm rounded to the nearest double, then truncated.  Values within
-// 1e-12 of an integer are taken as that integer (the correctly rounded
-// logarithm of a double nearest a power of ten is that integer).
-__device__ int nsig_of(double zeta) {
-  double L = -log10(fabs(zeta));
-  double k = rint(L);
-  int itmp = (fabs(L - k) <= 1e-12 * fmax(1.0, fabs(k))) ? (int)k : (int)L;
-  return itmp > 4 ? itmp : 4;
-}
-
-__device__ double pow10_neg(int nsig) {
-  double p = 1.0;
-  for (int i = 0; i < nsig; ++i) p *= 10.0;   // exact up to 1e22
-  return 1.0 / p;
-}
-
-// chgcon, jacobi case (itpackv.F:893-1027), for iteration `in`.  The
-// tridiagonal lives in the scalar block's shared memory (t1, t2).
-__device__ void chgcon_d(ItpLocal *it, double *t1, double *t2, int in) {
-  double start = it->cme, end1 = 0.0;
-  int ip = in;
-  if (ip == 0) {
-    it->cmold = 0.0;
-    it->cme = 0.0;
-    return;
-  }
-  if (ip == 1) {
-    end1 = 1.0 - 1.0 / it->gamma;
-    t1[0] = end1;
-    t2[0] = 0.0;
-    it->cme = end1;
-    return;
-  }
-  if (fabs(start - it->cmold) <= it->zeta * start) {
-    it->adapt = 0;
-    return;
-  }
-  it->cmold = start;
-  t1[ip - 1] = 1.0 - 1.0 / it->gamma;
-  t2[ip - 1] = (1.0 - it->rho) / (it->rho * it->rhoold * it->gamma * it->gamold);
-  int ier = 0;
-  if (it->isym != 0) {
-    ier = 903;
-  } else {
-    int nsig = nsig_of(it->zeta);
-    int maxfn = it->itmax > 50 ? it->itmax : 50;
-    double a = start, b = 1.0;
-    zbrent_d(ip, t1, t2, 0.0, pow10_neg(nsig), a, b, maxfn, ier);
-    end1 = b;
-  }
-  it->chg_ier = ier;
-  if (ier != 0) {
-    it->adapt = 0;
-    return;
-  }
-  it->cme = end1;
-}
-
 // ------------------------------------------------------------ row access
 // A row's off-diagonal slots are processed in chunks of kCh: the column and
 // value of every slot of the chunk are loaded first, then all neighbour
@@ -501,6 +342,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_kernel(JcgArgs a) {
     g->adapt = L.adapt; g->q1 = L.q1; g->chg_ier = L.chg_ier;
     g->in = fin;
     g->halt = h;
+    if (a.est) a.est->exact = 1;
     if (a.defer_drift == 1) *a.drift_pending = 1;
     a.flags->numitr = fin;
     a.flags->ier = (h == 2) ? 13 : 0;
@@ -628,6 +470,81 @@ int jcg_reset_exchange(adc_ctx *c) {
   return ADC_OK;
 }
 
+// What the last solve left undone of its estimate (have = false: nothing):
+// chgcon over the recorded coefficients, some 10 us for a solve of 20
+// iterations.  `head` and `pairs` are what the caller has copied of them
+// already.
+int jcg_estimate(const EstRec *est, cudaStream_t stream, Estimate &out, bool &have, const EstRec *head,
+                 const double2 *pairs, int npairs) {
+  have = false;
+  EstRec r;
+  if (head) {
+    r = *head;
+  } else {
+    ADC_CUDA(cudaMemcpyAsync(&r, est, sizeof(r), cudaMemcpyDeviceToHost, stream));
+    ADC_CUDA(cudaStreamSynchronize(stream));
+  }
+  if (r.exact || r.m < 0 || r.m > r.itmax) return ADC_OK;
+  std::vector<double2> all;
+  if (npairs < r.m) {
+    all.resize(r.m);
+    ADC_CUDA(cudaMemcpyAsync(all.data(), est + 1, r.m * sizeof(double2), cudaMemcpyDeviceToHost, stream));
+    ADC_CUDA(cudaStreamSynchronize(stream));
+    pairs = all.data();
+  }
+  std::vector<double> t1(r.m + 2), t2(r.m + 2);
+  ItpLocal L;
+  memset(&L, 0, sizeof(L));
+  L.zeta = r.zeta;
+  L.cme = r.cme0;
+  L.cmold = r.cmold0;
+  L.itmax = r.itmax;
+  L.adapt = r.adapt0;
+  for (int in = 0; in <= r.m && L.adapt; ++in) {
+    if (in > 0) {
+      L.gamma = pairs[in - 1].x;
+      L.rho = pairs[in - 1].y;
+    }
+    if (in > 1) {
+      L.gamold = pairs[in - 2].x;
+      L.rhoold = pairs[in - 2].y;
+    }
+    chgcon_d(&L, t1.data(), t2.data(), in);
+  }
+  out.serial = r.serial;
+  out.cme = L.cme;
+  out.cmold = L.cmold;
+  out.adapt = L.adapt;
+  out.ier = L.chg_ier;
+  out.stptst = L.cme != 1.0 ? r.sqd / (r.squd * (1.0 - L.cme)) : 1.0 / r.squd;   // pstop's tl / tr
+  have = true;
+  return ADC_OK;
+}
+
+// The step's flags, with the estimate of the last solve.
+int read_state(adc_ctx *c, Flags &f, Estimate &est, bool &have) {
+  constexpr int kPairs = 64;   // of most solves; more are copied apart
+  struct {
+    Flags f;
+    char words[kEstOffset - sizeof(Flags)];
+    EstRec r;
+    double2 pairs[kPairs];
+  } b;
+  const int n = std::min(kPairs, c->itmax + 2);
+  ADC_CUDA(cudaMemcpyAsync(&b, c->flags, kEstOffset + sizeof(EstRec) + n * sizeof(double2), cudaMemcpyDeviceToHost,
+                           c->stream));
+  ADC_CUDA(cudaStreamSynchronize(c->stream));
+  f = b.f;
+  est = c->est_last;
+  have = !b.r.exact && est.serial == b.r.serial;
+  if (!have) {
+    if (int rc = jcg_estimate(c->est, c->stream, est, have, &b.r, b.pairs, n)) return rc;
+    if (have) c->est_last = est;
+  }
+  if (have) f.cme = est.cme;
+  return ADC_OK;
+}
+
 int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int defer_drift, int d1) {
   JcgArgs a;
   a.do_peror = do_peror;
@@ -653,6 +570,7 @@ int launch_jcg_impl(adc_ctx *c, int eta_update, int do_peror, int run_init, int 
   a.bar = c->bar;
   a.arrive = c->jlines;
   a.flags = c->flags;
+  a.est = c->est;
   a.spin = c->spin_cycles > 0 ? c->spin_cycles : kSpinCycles;
   a.spin_mask = a.spin < 1000000 ? 0 : 63;   // 64 polls may take 100,000 cycles
   a.eta_update = eta_update;

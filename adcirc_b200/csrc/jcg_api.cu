@@ -140,6 +140,7 @@ static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, doubl
     st.place(&d_ell, (size_t)n * maxnz);
     st.place(&d_src, nnz);
     st.place(&d_state, 1);
+    st.place((char **)&c.est, sizeof(EstRec) + (itmax + 2) * sizeof(double2));
     st.place(&c.jtab_room, room);
     st.place((char **)&c.jlines, nlines);
     zero0 = (st.used + 255) & ~(size_t)255;   // from here on zeroed
@@ -191,6 +192,10 @@ static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, doubl
   if (it.zeta < temp) it.zeta = temp;
   it.rec.need_unorm = !it.q1;
   ADC_CUDA(up(d_state, &ss, sizeof(ss)));
+  EstRec er;
+  memset((void *)&er, 0, sizeof(er));
+  er.exact = 1;   // what a kernel other than the resident one leaves
+  ADC_CUDA(up(c.est, &er, sizeof(er)));
   rc = launch_jcg_impl(&c, 0, iparm[11] >= 0 ? 1 : 0, 0, 0, 0);
   if (rc) return rc;
   launch_k(k_slots_to_ell, std::max(1, nblk(nnz)), kThreads, c.stream, nnz, (const int *)d_src,
@@ -208,7 +213,13 @@ static int jcg_solve(int n, int ndim, int maxnz, int *jcoef, double *coef, doubl
   if (maxnz > 1)
     ADC_CUDA(cudaMemcpy2DAsync(coef + ndim, (size_t)ndim * sizeof(double), d_ell + n, n * sizeof(double),
                                n * sizeof(double), maxnz - 1, cudaMemcpyDeviceToHost, c.stream));
-  ADC_CUDA(cudaStreamSynchronize(c.stream));
+  Estimate est;
+  bool have;
+  if (int rc2 = jcg_estimate(c.est, c.stream, est, have)) return rc2;   // waits for the copies above
+  if (have) {
+    it.cme = est.cme;
+    it.stptst = est.stptst;
+  }
   g_q1 = it.q1;
   ier = fl.ier;
   in_out = it.in;

@@ -21,6 +21,7 @@ struct JcgArgs {
   Bar *bar;
   void *arrive;             // the barrier lines (see the kernels)
   Flags *flags;
+  EstRec *est;              // resident kernel: what the estimate's last value is formed from, if not here
   long long spin;           // cycles a wait may take ...
   unsigned spin_mask;       // ... and polls between looks at the clock and the timeout flag, less one
   int eta_update;

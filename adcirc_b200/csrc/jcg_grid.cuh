@@ -3,6 +3,7 @@
 // barrier that carries the dot products, and the serial scalar steps.
 #pragma once
 
+#include "jcg_chgcon.cuh"
 #include "jcg_common.cuh"
 
 namespace adc {
@@ -109,13 +110,6 @@ __device__ __forceinline__ unsigned long long pack_rec(const Rec &r) {
   return (unsigned long long)(unsigned)r.in | ((unsigned long long)(r.halt & 0xff) << 32) |
          ((unsigned long long)(r.need_unorm & 0xff) << 40);
 }
-
-// Serial ITPACK state of one solve, held in registers of the scalar block's
-// thread 0 (echall/itjcg/chgcon/pstop/parcon variables).
-struct ItpLocal {
-  double zeta, cme, gamma, rho, gamold, rhoold, delnnm, delsnm, udnm, stptst, cmold, rparm1;
-  int itmax, adapt, q1, isym, chg_ier;
-};
 
 // pstop_nrms (itpackv.F:809-890, iflag = 1) for iteration `in`.
 __device__ inline int pstop_d(ItpLocal *it, int in, double unrm, double dnrm) {

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
     if (warp != 0) return;
     double cme = L.cme, cmold = L.cmold;
     int adapt = L.adapt, ier = L.chg_ier;
-    if (adapt) chgcon_warp(L.gamma, L.rho, L.gamold, L.rhoold, L.zeta, ztol, a.itmax, tri, in, cme, cmold, adapt, ier);
+    if (adapt) chgcon_warp<true>(L.gamma, L.rho, L.gamold, L.rhoold, L.zeta, ztol, a.itmax, tri, in, cme, cmold, adapt, ier);
     __syncwarp();
     if (lane == 0) {
       L.cme = cme;
@@ -494,6 +494,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
     g->in = fin;
     g->halt = h;
     a.bar->gen = gen;
+    if (a.est) a.est->exact = 1;
     if (a.d1) a.flags->n_w1_events = 0;
     if (a.defer_drift == 1) *a.drift_pending = 1;
     a.flags->numitr = fin;

@@ -42,11 +42,16 @@
 // a timeout and all blocks return.
 //
 // The adaptive eigenvalue estimate (chgcon, :893-1027) feeds only the
-// stopping test.  The scalar warp of every block computes it from the
-// recorded parcon coefficients and may fall behind the row warps: the
-// estimate never decreases, so while the iterate's change is too large to
-// stop by an earlier estimate, it is too large by the exact one.  Only an
-// iteration for which that does not decide waits for its own estimate.
+// stopping test.  The scalar warp of every block forms bounds of it from the
+// recorded parcon coefficients (CmeBounds) and may fall behind the row warps:
+// the estimate never decreases, so while the iterate's change is too large to
+// stop by an earlier lower bound, it is too large by the exact estimate.  Only
+// an iteration for which that does not decide waits for its own bounds, and
+// only where the test falls between them does the scalar warp run chgcon
+// itself, from the first iteration on.  Run in every iteration, its search is
+// the longest chain of a solve on small meshes (6,500 cycles an iteration
+// beside the rows' 3,300 on a 4,961-node channel: 110 us a step for 75).  The
+// value that a caller sees is formed by jcg_estimate when it is asked for.
 //
 // u(m) is needed for its norm in the first iterations and then in every
 // fifth; in the others it is formed while the exchange is under way.
@@ -191,8 +196,8 @@ __device__ __forceinline__ double warp_sum_all(double v) {
 // The ITPACK scalars of one solve, in shared memory: parcon's stepped by
 // warp 0, pstop's by warp 1, read by the scalar warp.
 struct Scal {
-  double gamma, rho, gamold, rhoold, delnnm, delsnm, udnm, squd, tl, tr, con;
-  int q1, pad_;
+  double gamma, rho, gamold, rhoold, delnnm, delsnm, udnm, squd, sqd, tl, tr, con;
+  int q1, exact;
 };
 
 // What the other warps need of an iteration's serial step.
@@ -283,6 +288,29 @@ __device__ __forceinline__ double spmv_global(const uint4 *cv, const double *lv,
   return acc;
 }
 
+// chgcon as far as a scalar warp has run it, and on to iteration `to`; apart,
+// so that its registers and code do not lie in every solve's way.
+struct Chgcon {
+  double cme, cmold;
+  int in, adapt, ier;
+};
+static __device__ __forceinline__ void chgcon_to(Chgcon *c, int to, const double2 *hist, double2 *tri, double zeta,
+                                              double tol, int itmax) {
+  double cme = c->cme, cmold = c->cmold;
+  int in = c->in, adapt = c->adapt, ier = c->ier;
+  while (in < to) {
+    ++in;
+    if (!adapt) continue;
+    const double2 h = hist[max(in - 1, 0)], o = hist[max(in - 2, 0)];
+    chgcon_warp<false>(h.x, h.y, o.x, o.y, zeta, tol, itmax, tri, in, cme, cmold, adapt, ier);
+  }
+  c->cme = cme;
+  c->cmold = cmold;
+  c->in = in;
+  c->adapt = adapt;
+  c->ier = ier;
+}
+
 template <int K, int kGrid>
 __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a) {
   griddep_wait();
@@ -312,8 +340,11 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
   unsigned char *stage = sm + a.o_area + (size_t)(2 * warp) * a.stage_bytes;   // two buffers
   __shared__ Scal sc;
   __shared__ StepRec s_rec;
-  __shared__ double s_cme;                 // the scalar warp's estimate ...
-  __shared__ volatile int s_cme_m;         // ... and its iteration (-1: none yet)
+  __shared__ volatile double s_low, s_up;  // the scalar warp's bounds of the estimate ...
+  __shared__ volatile int s_cme_m;         // ... and their iteration (-1: none yet)
+  __shared__ volatile double s_con;        // the exact estimate, of the iteration
+  __shared__ volatile int s_exact_m;       // s_exact_m, where it is known or
+  __shared__ volatile int s_want;          // was asked for
   __shared__ volatile int s_hist;          // iterations recorded in hist
   __shared__ volatile int s_done;          // 1: the solve has ended, 2: a wait expired
   __shared__ int s_m;
@@ -585,7 +616,7 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
   if (tid == 0) {
     memset(&sc, 0, sizeof(sc));
     sc.q1 = q1_in;
-    s_cme_m = -1;
+    s_cme_m = s_exact_m = s_want = -1;
     s_hist = 0;
     s_done = 0;
   }
@@ -891,36 +922,58 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
             squd = sqrt(udnm);
           }
           const double sqd = sqrt(sd);
-          // an earlier estimate may decide: con(m) is no smaller, so that
-          // tr (1 - con) zeta is no larger (con = 1 does not stop either
-          // while squd zeta <= 1)
-          int h = 0;
-          const int seen = s_cme_m;
-          __threadfence_block();
-          const double low = *(volatile double *)&s_cme;
-          if (!(m >= 2 && seen >= 1 && m < a.itmax && squd * zeta <= 1.0 &&
-                sqd >= squd * (1.0 - low) * zeta)) {
+          // Waits of the scalar warp's; false where the wait expires.
+          const auto wait_for = [&](volatile int &at) {
             const long long tw = clock64();
-            while (s_cme_m < m) {
+            while (at < m) {
               if (clock64() - tw > a.spin) {
                 if (lane == 0) atomicExch(&a.flags->timeout, 1);
                 bad = 1;
-                break;
+                return;
               }
             }
             __threadfence_block();
-            const double con = *(volatile double *)&s_cme;
-            double tl = 1.0, tr = squd;
-            if (con != 1.0) {
-              tl = sqd;
-              tr = tr * (1.0 - con);
+          };
+          // an earlier lower bound may decide: con(m) is no smaller, so that
+          // tr (1 - con) zeta is no larger (con = 1 does not stop either
+          // while squd zeta <= 1)
+          const auto goes_on = [&](double low) {
+            return m < a.itmax && squd * zeta <= 1.0 && sqd >= squd * (1.0 - low) * zeta;
+          };
+          int h = 0;
+          const int seen = s_cme_m;
+          __threadfence_block();
+          if (!(m >= 2 && seen >= 1 && goes_on(s_low))) {
+            wait_for(s_cme_m);
+            bool exact = s_exact_m >= m;
+            if (!exact && !goes_on(s_low)) {
+              const double up = s_up;
+              if (m < a.itmax && up < 1.0 && sqd < squd * (1.0 - up) * zeta) {
+                h = 1;
+              } else {
+                if (lane == 0) s_want = m;
+                wait_for(s_exact_m);
+                exact = true;
+              }
             }
-            h = (tl >= tr * zeta) ? 0 : 1;
-            if (!h && m >= a.itmax) h = 2;
+            if (exact) {
+              const double con = s_con;
+              double tl = 1.0, tr = squd;
+              if (con != 1.0) {
+                tl = sqd;
+                tr = tr * (1.0 - con);
+              }
+              h = (tl >= tr * zeta) ? 0 : 1;
+              if (!h && m >= a.itmax) h = 2;
+              if (lane == 0) {
+                sc.tl = tl;
+                sc.tr = tr;
+                sc.con = con;
+              }
+            }
             if (lane == 0) {
-              sc.tl = tl;
-              sc.tr = tr;
-              sc.con = con;
+              sc.exact = exact;
+              sc.sqd = sqd;
             }
           }
           if (lane == 0) {
@@ -957,51 +1010,87 @@ __global__ void __launch_bounds__(kResThreads, 1) jcg_resident_kernel(JcgArgs a)
       need_u = s_rec.need_u;
     }
   } else {
-    double cmold = a.itp->cmold, cme = a.itp->cme;
+    const double cmold0 = a.itp->cmold, cme0 = a.itp->cme;
+    const int adapt0 = a.run_init ? 1 : a.itp->adapt;
     const double ztol = zbrent_tol(zeta);
-    int adapt = a.run_init ? 1 : a.itp->adapt, chg_ier = 0;
+    Chgcon ch = {cme0, cmold0, -1, adapt0, 0};
+    int ex = -1, adapt = adapt0;   // ch.in and ch.adapt
+    CmeBounds bd;
+    bd.low = bd.up = 0.0;
     // What the row warps have left in shared memory is read by lane 0 alone:
     // lanes that read it one by one may differ, and all of them go on together.
     int done = 0;   // s_done, where lane 0 last read it
-    for (int in = 0;; ++in) {
-      int go = 0;
+    for (int in = 0;;) {
+      int to = -1;   // run chgcon up to here; -2: the end
       if (lane == 0) {
         const long long tw = clock64();
-        while (s_hist < in && s_done == 0) {
+        while (s_hist < in && s_done == 0 && s_want <= ex) {
           if (clock64() - tw > 2 * a.spin) break;   // the row warps have given up before
         }
         done = s_done;
-        go = s_hist >= in && (in == 0 || done == 0);
+        if (in > 0 && done != 0) to = -2;
+        else if (s_want > ex) to = s_want;
+        else if (s_hist < in) to = -2;
         __threadfence_block();
       }
-      go = __shfl_sync(0xffffffffu, go, 0);
+      to = __shfl_sync(0xffffffffu, to, 0);
       __syncwarp();   // lane 0's reads before every lane's
-      if (!go) break;
-      if (adapt) {
-        const double2 h = hist[max(in - 1, 0)], o = hist[max(in - 2, 0)];
-        chgcon_warp(h.x, h.y, o.x, o.y, zeta, ztol, a.itmax, tri, in, cme, cmold, adapt, chg_ier);
+      if (to == -2) break;
+      // the first two, and all once the estimate stays as it is, cost nothing
+      const bool next = to < 0;
+      if (next && ex == in - 1 && (in <= 1 || !adapt)) to = in;
+      if (ex < to) {
+        chgcon_to(&ch, to, hist, tri, zeta, ztol, a.itmax);
+        ex = to;
+        adapt = ch.adapt;
+      }
+      if (next) {
+        if (ex == in) {
+          if (in == 1) bd.start(zeta, s_con, ch.cme);
+          else bd.low = bd.up = ch.cme;
+        } else {
+          const double2 h = hist[in - 1], o = hist[in - 2];
+          tri_entries(h.x, h.y, o.x, o.y, tri, in);
+          bd.next(zeta, ztol, tri, in);
+        }
       }
       if (lane == 0) {
-        s_cme = cme;
-        __threadfence_block();
-        s_cme_m = in;
+        if (ex == to) {
+          s_con = ch.cme;
+          __threadfence_block();
+          s_exact_m = ex;
+        }
+        if (next) {
+          s_low = bd.low;
+          s_up = bd.up;
+          __threadfence_block();
+          s_cme_m = in;
+        }
       }
       __syncwarp();
+      if (next) ++in;
     }
     ended = __shfl_sync(0xffffffffu, done, 0) == 1;
     m = s_m;
+    if (ended && b == 0 && !sc.exact)
+      for (int k = lane; k < m; k += 32) ((double2 *)(a.est + 1))[k] = hist[k];
     if (ended && b == 0 && lane == 0) {
       const Scal s = sc;
       const int halt = s_rec.halt;
-      const double stptst = s.tl / s.tr;
+      const double stptst = s.exact ? s.tl / s.tr : 0.0;
       double rparm1 = a.itp->rparm1;
       if (halt == 2) rparm1 = stptst;   // itpackv.F:394
+      // without the exact estimate, jcg_estimate's inputs
+      EstRec *er = a.est;
+      er->zeta = zeta; er->cme0 = cme0; er->cmold0 = cmold0; er->sqd = s.sqd; er->squd = s.squd;
+      er->m = m; er->itmax = a.itmax; er->adapt0 = adapt0; er->exact = s.exact;
+      ++er->serial;
       Itp *g = a.itp;
       g->zeta = zeta; g->cme = s.con; g->gamma = s.gamma; g->rho = s.rho;
       g->gamold = s.gamold; g->rhoold = s.rhoold; g->delnnm = s.delnnm; g->delsnm = s.delsnm;
-      g->udnm = s.udnm; g->stptst = stptst; g->cmold = cmold; g->rparm1 = rparm1;
+      g->udnm = s.udnm; g->stptst = stptst; g->cmold = ch.cmold; g->rparm1 = rparm1;
       g->sme = -1.0; g->itmax = a.itmax; g->isym = 0;
-      g->adapt = adapt; g->q1 = s.q1; g->chg_ier = chg_ier;
+      g->adapt = adapt; g->q1 = s.q1; g->chg_ier = ch.ier;
       g->in = m;
       g->halt = halt;
       if (a.defer_drift == 1) *a.drift_pending = 1;

@@ -557,10 +557,13 @@ static int bind_impl(const adc_params_t *p, const adc_arrays_t *a, int prec, adc
   B(dalloc((char **)&c->jlines, 2 * 128 * (size_t)c->jcg_rows_blocks));
   jcg_clear_barrier(c);
   {
-    // Flags followed by the rebuild word.
+    // Flags, the LHS words and tickets, and the estimate's record.
     char *f = nullptr;
-    if (cudaMalloc((void **)&f, sizeof(Flags) + 64) != cudaSuccess) return fail(ADC_ERR_NOMEM);
+    const size_t bytes = kEstOffset + sizeof(EstRec) + (c->itmax + 2) * sizeof(double2);
+    if (cudaMalloc((void **)&f, bytes) != cudaSuccess) return fail(ADC_ERR_NOMEM);
+    if (cudaMemset(f, 0, bytes) != cudaSuccess) return fail(ADC_ERR_CUDA);
     c->flags = (Flags *)f;
+    c->est = (EstRec *)(f + kEstOffset);
     c->tickets = (int *)(c->flags + 1) + 4;   // after the four LHS words
   }
   c->steps_cap = 1;
@@ -583,6 +586,10 @@ static int bind_impl(const adc_params_t *p, const adc_arrays_t *a, int prec, adc
   B(up(c->flags, &fl, 1));
   int words[6] = {0, 0, 0, 1, 0, 0};   // rebuild, drift pending/applied, gather every row, tickets
   B(up(rebuild_flag(c), words, 6));
+  EstRec er;
+  memset((void *)&er, 0, sizeof(er));
+  er.exact = 1;
+  B(up(c->est, &er, 1));
   ADC_CUDA(cudaDeviceSynchronize());
 #undef B
   *out = c;
@@ -590,8 +597,9 @@ static int bind_impl(const adc_params_t *p, const adc_arrays_t *a, int prec, adc
 }
 
 static int read_flags(adc_ctx *c, Flags &f) {
-  ADC_CUDA(cudaMemcpyAsync(&f, c->flags, sizeof(Flags), cudaMemcpyDeviceToHost, c->stream));
-  ADC_CUDA(cudaStreamSynchronize(c->stream));
+  Estimate est;
+  bool have;
+  TRY(read_state(c, f, est, have));
   if (f.timeout) { set_error("a bounded device-side wait expired"); return ADC_ERR_TIMEOUT; }
   return ADC_OK;
 }
@@ -833,7 +841,7 @@ int adc_get_scalars(adc_ctx *c, adc_scalars_t *out) {
   out->q1 = it.q1;
   out->ep = f.ep;
   out->rparm1 = it.rparm1;
-  out->rparm2 = it.cme;
+  out->rparm2 = f.cme;
   out->vortex_counter = -1;
   out->vortex_wtratio = 0.0;
   if (c->vortex_on) {

@@ -83,3 +83,42 @@ def test_many_iterations(lib, nx, eps, zeta):
     o = _solve((orc.orc_jcg, orc.orc_dfault, orc.orc_itpack_reset), *sysargs, zeta, itmax=1400)
     assert g[:2] == o[:2] and o[1] >= 400
     assert abs(g[2] - o[2]) <= 1e-12
+
+
+def test_estimate_of_steps(lib, orc, tmp_path):
+    """The estimate that adc_timestep, adc_gwce_new, adc_run, adc_get_scalars
+    and a dump report is the oracle's of the same solve, though the solve has
+    stopped by bounds of it; after a dump is read back too."""
+    import ctypes as C
+
+    from adcirc_b200 import _lib, model
+    case0, case = model.channel_case(prep=orc.mesh_prep()), model.channel_case()
+    om, gm = orc.OracleModel(case0), model.GpuModel(case)
+    want = [om.step(it).cme for it in range(1, 13)]
+
+    def same(x, y):
+        return abs(x - y) <= 1e-12 * max(abs(y), 1.0)
+
+    for it in range(1, 5):
+        assert same(gm.step(it).cme, want[it - 1]), it
+        assert same(gm.scalars()["rparm2"], want[it - 1]), it
+    out = _lib.AdcStepOut()
+    for it in (5, 6):
+        s = C.byref(case.schedule.step(it))
+        assert lib.adc_shift_friction(gm.h, s) == 0
+        assert lib.adc_gwce_new(gm.h, s, C.byref(out)) == 0
+        assert same(out.cme, want[it - 1]), it
+        assert lib.adc_wetdry(gm.h, s, C.byref(out)) == 0
+        assert same(out.cme, want[it - 1]), it
+        assert lib.adc_momentum(gm.h, s) == 0
+    _, last = gm.run(7, 3)
+    assert same(last.cme, want[8])
+    gm.hotstart_write(tmp_path / "a")
+    gm.run(10, 3)
+    assert same(gm.scalars()["rparm2"], want[11])
+    gm.hotstart_read(tmp_path / "a")
+    assert same(gm.scalars()["rparm2"], want[8])
+    gm.hotstart_write(tmp_path / "b")
+    assert (tmp_path / "a").read_bytes() == (tmp_path / "b").read_bytes()
+    gm.close()
+    om.close()
