@@ -215,8 +215,6 @@ struct adc_ctx {
   // JCG
   double *ju1, *jw, *soff;
   double4 *jp[2];        // JCG (dtwd, d, d_prev, -) per node, double-buffered
-  double *jpart;         // partial dots per block (4 each)
-  double *jtri;          // tri(itmax,4)
   adc::Itp *itp;
   adc::Bar *bar;
   void *jlines;          // JCG barrier lines: 2 x 128 B per row block
@@ -236,7 +234,7 @@ struct adc_ctx {
   uint4 *jrcol;
   int4 *jmeta;
   unsigned char *jrle;
-  float *soff32;               // FP32 scaled matrix (mixed mode, resident variant)
+  float *soff32;               // FP32 scaled matrix (mixed mode)
   double *etas_prev;           // last step's reference guess (ADC_WARM_START)
   WarmState *warm;
   adc::Mpnn *mp;               // learned initial guess (mpnn.cu), built on first use

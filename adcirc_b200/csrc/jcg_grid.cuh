@@ -105,12 +105,6 @@ __device__ inline Rec read_rec(const Rec *r) {
   return o;
 }
 
-// The record's integers in one word (never kEmpty: the top 16 bits are 0).
-__device__ __forceinline__ unsigned long long pack_rec(const Rec &r) {
-  return (unsigned long long)(unsigned)r.in | ((unsigned long long)(r.halt & 0xff) << 32) |
-         ((unsigned long long)(r.need_unorm & 0xff) << 40);
-}
-
 // pstop_nrms (itpackv.F:809-890, iflag = 1) for iteration `in`.
 __device__ inline int pstop_d(ItpLocal *it, int in, double unrm, double dnrm) {
   double con = it->cme, uold, tr, tl;

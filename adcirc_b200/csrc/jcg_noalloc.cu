@@ -97,8 +97,10 @@ static void noalloc_carve(Carve &cv, adc_ctx &c, int n, int nslices, size_t slot
   c.jw = cv.take<double>(npad);
   c.jp[0] = cv.take<double4>(npad);
   c.jp[1] = cv.take<double4>(npad);
-  c.jpart = cv.take<double>(4 * (size_t)c.jcg_grid);
-  c.jtri = cv.take<double>(4 * (size_t)(itmax > 2 ? itmax : 2));
+  // in no kernel's use, but part of the capacity that callers are told: a
+  // system is taken or refused (905) by the same count as ever
+  cv.take<double>(4 * (size_t)c.jcg_grid);
+  cv.take<double>(4 * (size_t)(itmax > 2 ? itmax : 2));
   c.jlines = cv.take<char>(2 * 128 * (size_t)c.jcg_rows_blocks);
   c.itp = cv.take<Itp>(1);
   c.bar = cv.take<Bar>(1);

@@ -32,7 +32,7 @@ constexpr int kRowUnroll = 8;   // rows per thread whose loads issue together
 constexpr int kHaloPre = 2;     // halo records per thread fetched ahead of the row update
 
 // Per-warp double-buffered bulk copies of whole slices (block-local
-// columns + one value array) into shared memory, for the resident variant.
+// columns + one value array) into shared memory.
 // Every copy that is issued is waited for before the next phase.
 struct SlicePipe {
   unsigned char *stg0;        // this warp's two buffers
@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
   const int n = a.n;
   const int r0 = s0 * kSlice, rows = (s1 - s0) * kSlice;   // the block's rows [r0, r0 + rows)
   extern __shared__ __align__(128) unsigned char s_dyn[];
-  // Dynamic shared memory.  Scalar block: the CG tridiagonal.  Row blocks
-  // of the resident variant: dtwd of the block's rows; two value buffers
+  // Dynamic shared memory.  Scalar block: the CG tridiagonal.  Row blocks:
+  // dtwd of the block's rows; two value buffers
   // (d of the rows, then the halo's new d) that trade roles every
   // iteration; per row its length and export bit; the slice table; one
   // mbarrier and two staging buffers per warp.
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
 
   const int need_u0 = !q1;   // the norm of u at iteration 0
   double pd = 0.0, pt = 0.0, pu = 0.0;
-  // Resident prologue.  Shared memory first holds, per row of the block
+  // Prologue.  Shared memory first holds, per row of the block
   // and per halo node, w = 1/sqrt(diag) and u' (P1), then d0 (P2).
   double *Uv = S_dd, *Wv = S_dd + VB;
   if (!scalar_block) {
@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
   // norms of iteration in+1.  P[in % 2][i] = (dtwd(in), d(in), d(in-1)) so
   // a neighbour's three values arrive in one 32-byte sector.
   P4 *P[2] = {p0, p1};
-  // u(in) and u(in-1): the resident prologue leaves u' in u1 and zeroes u
+  // u(in) and u(in-1): the prologue leaves u' in u1 and zeroes u
   double *U[2] = {a.u1, a.u};
-  int cur = 0;   // resident variant: S_dd half holding d(in)
+  int cur = 0;   // S_dd half holding d(in)
   for (int in = 0; in < a.itmax; ++in) {
     const Rec r = s_rec;
     if (r.halt) break;
@@ -368,8 +368,7 @@ __global__ void __launch_bounds__(kThreads, 2) jcg_ordered_kernel(JcgArgs a) {
     double *un = U[(in + 1) % 2];
     double pd = 0.0, pt = 0.0, pu = 0.0;
     if (!scalar_block) {
-      // Resident variant.  The warp's first two slices start streaming
-      // before phase A.
+      // The warp's first two slices start streaming before phase A.
       pipe.begin((const VT *)sv_store, false);   // unchanged since P2's fence
       // Phase A: the 3-term update of the block's rows, d(in+1) written
       // over d(in-1); then the new d of the halo nodes from their owners'
@@ -509,7 +508,7 @@ static size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 static size_t jcg_stage_bytes(int wmax) { return round_up((size_t)std::max(wmax, 1) * 320, 128); }
 
 // Dynamic shared memory of one block (the largest of the scalar block's
-// tridiagonal and a resident row block's layout, see jcg_kernel).
+// tridiagonal and a row block's layout, see the kernel).
 static size_t jcg_smem_bytes(int itmax, int rows_max, int halo_max, int wmax) {
   size_t tri = round_up(sizeof(double2) * (itmax + 2), 128);
   size_t rb = (size_t)rows_max, vb = rb + (size_t)halo_max;
@@ -522,7 +521,7 @@ static int jcg_row_block_begin(int nslices, int nrb, int b) {
   return (int)((long long)nslices * b / nrb);
 }
 
-// Block-local column indices of the resident variant.  Row block b owns the
+// Block-local column indices.  Row block b owns the
 // rows of slices [s0, s1); a neighbour in that range maps to its offset
 // from the block's first row, any other neighbour to rows_max + its
 // position in the block's halo list (first appearance in slot order).

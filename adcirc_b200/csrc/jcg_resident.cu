@@ -130,9 +130,6 @@ __device__ __forceinline__ uint32_t cluster_addr(const void *p, int rank) {
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
 __device__ __forceinline__ double ld_cluster(uint32_t a) {
   double v;
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");

@@ -766,9 +766,9 @@ static int launch_predictor_backward(adc_ctx *c) {
   return ADC_OK;
 }
 
-// Training step: backpropagation, then Adam and the BF16 weight copies.
 bool predictor_trains(const adc_ctx *c) { return c->mp && c->mp->train; }
 
+// Training step: backpropagation, then Adam and the BF16 weight copies.
 int launch_predictor_train(adc_ctx *c) {
   Mpnn *mp = c->mp;
   if (!mp || !mp->train) return ADC_OK;

@@ -1,10 +1,8 @@
 // step_bodies.cuh -- the 2DDI step (timestep.F, gwce.F, wetdry.F,
 // momentum.F, nws08.F90) item by item: what one node, element, boundary entry
-// or warp of elements does in each pass.  The grid kernels (gwce.cu, met.cu,
-// flux.cu, wetdry.cu, momentum.cu) run a pass over a whole mesh; the cluster
-// kernels (step_small.cu) run all passes of a small mesh between cluster
-// barriers.  Every pass keeps the reference's operations and, per node, its
-// element order.
+// or warp of elements does in each pass.  The kernels (gwce.cu, flux.cu,
+// wetdry.cu, momentum.cu) run a pass over the mesh.  Every pass keeps the
+// reference's operations and, per node, its element order.
 #pragma once
 
 #include "adc_internal.cuh"
@@ -799,14 +797,11 @@ __device__ __forceinline__ double hyb_term(const adc_params_t &p, double h1) {
 constexpr int kW1Block = 256;
 constexpr int kChainFast = 1024;   // W1 events resolved in shared memory at a time
 
-// W1, wetdry.F:332-809, plus NOFFOLD/NOFF initialisation (:222-225), for G
-// consecutive blocks of 256 elements from vb0, one per 256 threads of the
-// thread block.
-template <int G>
-__device__ __forceinline__ void block_w1(const adc_ctx &c, int vb0) {
-  const int grp = (int)threadIdx.x / kW1Block, t = (int)threadIdx.x % kW1Block;
-  const int vb = vb0 + grp;   // this group's block of elements
-  const int e = vb < c.ev_blocks ? vb * kW1Block + t : c.ne;
+// W1, wetdry.F:332-809, plus NOFFOLD/NOFF initialisation (:222-225), for the
+// vb-th block of 256 elements.
+__device__ __forceinline__ void block_w1(const adc_ctx &c, int vb) {
+  const int t = (int)threadIdx.x;
+  const int e = vb * kW1Block + t;
   bool ev = false;
   int ea = 0, eb = 0;
   double ec = 0.0;
@@ -851,22 +846,22 @@ __device__ __forceinline__ void block_w1(const adc_ctx &c, int vb0) {
     }
   }
   // block-local ordered compaction of the events
-  __shared__ int wcnt[G][kW1Block / 32];
+  __shared__ int wcnt[kW1Block / 32];
   unsigned m = __ballot_sync(0xffffffffu, ev);
   const int lane = t & 31, w = t >> 5;
-  if (lane == 0) wcnt[grp][w] = __popc(m);
+  if (lane == 0) wcnt[w] = __popc(m);
   __syncthreads();
   int off = 0, tot = 0;
   for (int k = 0; k < kW1Block / 32; ++k) {
-    if (k < w) off += wcnt[grp][k];
-    tot += wcnt[grp][k];
+    if (k < w) off += wcnt[k];
+    tot += wcnt[k];
   }
   // each event goes to its block's ordered slot and, while the step has at
   // most kChainFast events, to an unordered list tagged with its element
-  __shared__ int s_ubase[G];
-  if (t == 0 && vb < c.ev_blocks) {
+  __shared__ int s_ubase;
+  if (t == 0) {
     c.ev_cnt[vb] = tot;
-    s_ubase[grp] = tot ? atomicAdd(&c.flags->n_w1_events, tot) : 0;
+    s_ubase = tot ? atomicAdd(&c.flags->n_w1_events, tot) : 0;
   }
   __syncthreads();
   if (ev) {
@@ -875,7 +870,7 @@ __device__ __forceinline__ void block_w1(const adc_ctx &c, int vb0) {
     c.ev_a[pos] = ea;
     c.ev_b[pos] = eb;
     c.ev_c[pos] = ec;
-    const int u = s_ubase[grp] + r;
+    const int u = s_ubase + r;
     if (u < kChainFast) {
       c.evu_i[3 * u] = ea;
       c.evu_i[3 * u + 1] = eb;

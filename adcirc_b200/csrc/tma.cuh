@@ -50,12 +50,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Orders this thread's generic-proxy global accesses with later async-proxy
-// (bulk copy) accesses to the same memory.
-__device__ __forceinline__ void fence_proxy_async_global() {
-  asm volatile("fence.proxy.async.global;" ::: "memory");
-}
-
 // Orders this thread's earlier generic-proxy accesses (shared and global,
 // including what it acquired from other threads) with its later bulk copies.
 __device__ __forceinline__ void fence_proxy_async_all() {

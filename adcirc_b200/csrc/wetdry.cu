@@ -24,7 +24,7 @@ __global__ void k_wd_d1(adc_ctx c) {
 
 __global__ void __launch_bounds__(kW1Block) k_wd_w1(adc_ctx c) {
   griddep_wait();
-  block_w1<1>(c, blockIdx.x);
+  block_w1(c, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(1024) k_wd_chain(adc_ctx c) {

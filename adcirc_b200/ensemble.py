@@ -129,9 +129,11 @@ class Ensemble:
 
 
 def candidate_layouts(sizes, sm_count: int = 148):
-    """JCG row blocks per member: each member's own default (0), and
-    shares of one or two blocks per SM split in proportion to member size
-    (every member at least one block)."""
+    """JCG row blocks per member: each member's own default (0), and shares of
+    the SMs in proportion to member size (every member at least one block):
+    of one block an SM, which is what the FP64 kernel with its vectors on the
+    SMs takes, and of two, for the kernels of the modes with FP32 parts and of
+    members too large for their share.  Only the default may be a cluster."""
     sizes = np.asarray(sizes, np.float64)
     cands = {"default": [0] * len(sizes)}
     for name, total in (("share_1x", sm_count), ("share_2x", 2 * sm_count - len(sizes))):

@@ -625,8 +625,10 @@ int adc_phase_times(adc_ctx *ctx, double *ms_shift, double *ms_gwce, double *ms_
 int adc_kernel_times(adc_ctx *ctx, double *ms, int n);
 
 /* JCG launch shape of a bound context (no reference counterpart): the
- * persistent solver's row blocks (0 restores the default choice) and
- * whether the resident variant (row vectors in shared memory) is used.
+ * persistent solver's row blocks (0 restores the default choice, the only
+ * one that may be a thread-block cluster) and whether a kernel with
+ * block-local tables and its vectors on the SMs is used: in FP64 one block
+ * an SM as far as that goes, else, and with FP32 parts, two.
  * adc_set_jcg_blocks rebuilds the solver's tables; results do not depend
  * on it beyond the dot products' summation tree. */
 int adc_set_jcg_blocks(adc_ctx *ctx, int row_blocks);
