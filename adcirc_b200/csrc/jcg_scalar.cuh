@@ -91,7 +91,12 @@ __device__ inline int tri_root_warp(int n, const double2 *tri, double lo, double
   for (int round = 0; round < 60; ++round) {
     const double f = tri_det(n, tri, x);
     const double flo = __shfl_sync(0xffffffffu, f, 0), fhi = __shfl_sync(0xffffffffu, f, 31);
-    if (round == 0 && ((flo > 0.0 && fhi > 0.0) || (flo < 0.0 && fhi < 0.0))) return 502;
+    if (round == 0) {
+      // no value may run out of range beside the root, where zbrent would take
+      // it for the root itself (hundreds of rows)
+      if (!(rcp_range(flo) && rcp_range(fhi))) return 501;
+      if ((flo > 0.0) == (fhi > 0.0)) return 502;
+    }
     const bool hit = f == 0.0 || (fhi > 0.0 ? f > 0.0 : f < 0.0);
     const unsigned m = __ballot_sync(0xffffffffu, hit);
     if (m & 1u) {   // the lower end itself is the root
