@@ -143,11 +143,29 @@ class ClockSampler:
 # Algorithmic bytes per launch (what each roofline's `achieved` is built on)
 # ----------------------------------------------------------------------------
 
-def jcg_bytes(nnz_o: int, npn: int, iters: float, vbytes: int = 8) -> float:
-    """Algorithmic HBM bytes of one JCG solve (persistent kernel), counted
-    as a streaming implementation would move them.
+def jcg_kernel_name(models, chosen: str, mode: int) -> str:
+    """The solver kernel of the chosen path's context (csrc/jcg.cu)."""
+    import ctypes as C
+    import torch
+    g, _ = models[chosen]
+    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    rb, res = C.c_int(0), C.c_int(0)
+    g.lib.adc_jcg_layout(g.h, C.byref(rb), C.byref(res))
+    if not res.value:
+        return "jcg_kernel"
+    return "jcg_ordered_kernel" if mode & 29 or rb.value > sms else "jcg_resident_kernel"
 
-    Per off-diagonal slot: the scaling pass, which also forms d0, reads the
+
+def jcg_bytes(kernel: str, nnz_o: int, npn: int, iters: float, vbytes: int = 8) -> float:
+    """Algorithmic HBM bytes of one JCG solve (persistent kernel).
+
+    jcg_resident_kernel, whose iterations work on chip: the matrix once, value
+    and column (12 B per off-diagonal slot); per row diagonal, guess and load
+    vector read (24 B), w and load vector written (16), the epilogue's w, ETA1,
+    NODECODE and DP read (28), solution, diagonal and ETA2 written (24).
+
+    The other two, as a streaming implementation would move them.  Per
+    off-diagonal slot: the scaling pass, which also forms d0, reads the
     FP64 value + column and writes the scaled value (vbytes: 8, or 4 for the
     FP32 matrix copy); each later SpMV pass (dtwd0, one per iteration) reads
     value + 4 B column.
@@ -155,6 +173,8 @@ def jcg_bytes(nnz_o: int, npn: int, iters: float, vbytes: int = 8) -> float:
     u1 16, row length 4, writes 32+8 minus the neighbours' records counted
     once), epilogue 60 B.
     """
+    if kernel == "jcg_resident_kernel":
+        return 12.0 * nnz_o + 92.0 * npn
     slot = vbytes + 4.0
     return (nnz_o * (12.0 + vbytes + slot * (1.0 + iters)) +
             npn * (64.0 + 44.0 + 24.0 + 68.0 * iters + 60.0))
@@ -167,7 +187,9 @@ def kernel_bytes(npn: int, ne: int, f32_mom: bool = False) -> dict:
                (156 B); per element: NM 12 + FDXE/FDYE 48 + AREAS 8 + ALPHAL
                8 + NOFF 4 (80 B) and three FP64 contributions written (24 B).
     rhs_gather per node: CSR pointer 4 + GWCE_LV write 8 + 40 B of nodal
-               I/O; per element-vertex entry: index 4 + contribution 8.
+               I/O; per element-vertex entry: index 4 + contribution 8.  The
+               matrix rows that a rebuild gathers in the same kernel vary with
+               the front and are not counted.
     mom_elem   per node: 12 gathered FP64 nodal fields + NODECODE (100 B);
                per element: 80 B element data + 6 contributions (48 B, or
                24 B in FP32).
@@ -516,6 +538,7 @@ def bench_gpu(args, rank, world, dist):
     import ctypes as C
     h2d = HOUR_STEPS * C.sizeof(_lib.AdcStep)
     d2h = HOUR_STEPS * C.sizeof(_lib.AdcStepOut) + sync_bytes
+    jcg_name = jcg_kernel_name(models, chosen, PATHS[chosen][0])
     for g, _ in models.values():
         g.close()
     # rooflines
@@ -526,7 +549,7 @@ def bench_gpu(args, rank, world, dist):
     mode = PATHS[chosen][0]
     vb = 4 if mode & 9 else 8
     kb = kernel_bytes(npn, ne, f32_mom=bool(mode & 17))
-    jb = jcg_bytes(nnz_o, npn, mean_it, vbytes=vb)
+    jb = jcg_bytes(jcg_name, nnz_o, npn, mean_it, vbytes=vb)
     rl = {}
     for k, nbytes in [("jcg", jb)] + list(kb.items()):
         ms = kt_sum.get(k, 0.0)
@@ -559,7 +582,9 @@ def bench_gpu(args, rank, world, dist):
         "ensemble": ens,
         "jcg_iters_per_step": res[chosen]["jcg_iters_per_step"],
         "kernel_ms": kt_sum,
-        "roofline": {"bound": "hbm", "kernel": "jcg_kernel", "achieved": rl["jcg"]["achieved_gbs"],
+        "roofline": {"bound": "latency (one exchange over the grid and one pass over the SMs' shared "
+                              "memory per iteration); the rate is of HBM",
+                     "kernel": jcg_name, "achieved": rl["jcg"]["achieved_gbs"],
                      "peak": peak, "unit": "GB/s", "frac": rl["jcg"]["frac"], "traffic": None,
                      "traffic_note": "DRAM bytes per launch come from an ncu capture, summarised "
                                      "in profiles/", "peak_kind": peak_kind,
